@@ -149,7 +149,7 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
   __shared__ __align__(8) unsigned long long barriers[2 * stages + 4];
   __shared__ uint32_t tmem_base_slot;
   __shared__ unsigned long long row_best[mode == 2 ? padded_rows : 1];
-  __shared__ int epilogue_gave_up;   // modes 2, 3: set by an epilogue warp whose wait ran out
+  __shared__ int epilogue_gave_up;   // mode 3: set by an epilogue warp whose wait ran out
   __shared__ int tail_is_last;       // mode 3: this CTA finished the last K piece of a tail tile
   __shared__ __align__(16) __nv_bfloat16 exchange[mode == 3 ? 2 * 128 * 16 : 8];
 
@@ -351,7 +351,7 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
         atomicExch(args.device_error, 3);
         epilogue_gave_up = 1;
       }
-      if constexpr (mode == 2 || mode == 3) {
+      if constexpr (mode == 3) {
         // The four epilogue warps meet at a named barrier further down, so they must leave the
         // loop together: each one's wait is bounded, all reach this barrier, and all read the
         // same flag after it.
@@ -469,19 +469,18 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
       if (lane == 0)
         ptx::mbarrier_arrive(acc_empty_bar + 8U * buffer);
       }
-
-      if constexpr (mode == 2) {
-        {
-          // Combine the four feature quarters in shared memory, then one global atomic per row.
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          for (int row = epilogue_thread; row < args.rows && row < padded_rows; row += 128) {
-            const unsigned long long candidate = row_best[row];
-            if (candidate != 0ULL)
-              atomicMax(args.best + row, candidate);
-            row_best[row] = 0ULL;
-          }
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
+    }
+    if constexpr (mode == 2) {
+      // Every tile of this CTA is in row_best: one global atomic per row and CTA. One per tile and
+      // row kept the L2 slice of the few key lines busy all through the launch, and whatever
+      // else lived in that slice (activation lines, by their addresses) waited behind it: the
+      // drafter's head (24 x 1024 x 262144, 2048 tiles) took 86 us or 150 to 190 by where its
+      // inputs lay, and takes 86 to 88 now (6.1 TB/s).
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      for (int row = epilogue_thread; row < args.rows && row < padded_rows; row += 128) {
+        const unsigned long long candidate = row_best[row];
+        if (candidate != 0ULL)
+          atomicMax(args.best + row, candidate);
       }
     }
     if constexpr (mode == 3) {
