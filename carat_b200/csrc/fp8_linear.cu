@@ -14,7 +14,9 @@
 #include "fp8_linear.cuh"
 #include "context.cuh"
 #include "launch.cuh"
+#include "linear_epilogue.cuh"
 #include "linear_items.cuh"
+#include "pair_linear.cuh"
 #include "ptx.cuh"
 #include "row_ops.cuh"
 
@@ -36,52 +38,17 @@ __host__ __device__ constexpr int stages_for(int padded_rows) {
   return fit > 8 ? 8 : fit;
 }
 
-__device__ __forceinline__ unsigned int orderable_bf16(float rounded) {
-  // Monotonic map of a bf16-representable float to 16 bits; NaN sorts below everything, matching
-  // a comparison chain that never selects NaN.
-  if (rounded != rounded)
-    return 0U;
-  const unsigned int bits = __float_as_uint(rounded) >> 16;
-  return (bits & 0x8000U) ? (~bits & 0xFFFFU) : (bits | 0x8000U);
-}
-
 // Finishes 32 accumulator columns (activation rows chunk*32 ..) of one feature.
-template <int mode>
 __device__ __forceinline__ void finish_chunk(const KernelArguments &args, const float (&values)[32],
-                                             int chunk, int feature, int feature_base, int lane,
-                                             float scale, unsigned long long *row_best) {
-  if constexpr (mode == 0) {
-    if (feature < args.output_width) {
-#pragma unroll
-      for (int column = 0; column < 32; ++column) {
-        const int row = chunk * 32 + column;
-        if (row < args.rows)
-          args.output[static_cast<size_t>(row) * args.output_width + feature] =
-              __float2bfloat16_rn(values[column] * scale);
-      }
-    }
-  } else {
-    unsigned long long chunk_best = 0ULL;
+                                             int chunk, int feature, float scale) {
+  if (feature < args.output_width) {
 #pragma unroll
     for (int column = 0; column < 32; ++column) {
-      const float rounded = __bfloat162float(__float2bfloat16_rn(values[column] * scale));
-      // Out-of-range features lose to everything; ties inside the warp go to the lowest lane,
-      // which is the lowest feature index.
-      const unsigned int key =
-          feature < args.output_width
-              ? ((orderable_bf16(rounded) + 1U) << 8) | static_cast<unsigned int>(31 - lane)
-              : 0U;
-      const unsigned int winner = __reduce_max_sync(0xFFFFFFFFU, key);
-      if (lane == column && winner != 0U) {
-        const unsigned int winner_feature =
-            static_cast<unsigned int>(feature_base) + (31U - (winner & 31U));
-        chunk_best = (static_cast<unsigned long long>(winner >> 8) << 32) |
-                     static_cast<unsigned long long>(~winner_feature);
-      }
+      const int row = chunk * 32 + column;
+      if (row < args.rows)
+        args.output[static_cast<size_t>(row) * args.output_width + feature] =
+            __float2bfloat16_rn(values[column] * scale);
     }
-    const int row = chunk * 32 + lane;
-    if (row < args.rows && chunk_best != 0ULL)
-      atomicMax(&row_best[row], chunk_best);
   }
 }
 
@@ -433,9 +400,12 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
                       __uint_as_float(raw[column]);
               }
             }
+          } else if constexpr (mode == 2) {
+            argmax_chunk(raw, scale, feature, feature_base, args.output_width, lane, chunk * 32,
+                         args.rows, row_best);
           } else {
             bool finished = false;
-            if constexpr (mode == 0) {
+            {
               if (item.tail) {    // warp-uniform
                 const int tail_width = args.tail_tiles * tile_features;
                 const int tail_feature = feature - (args.tiles - args.tail_tiles) * tile_features;
@@ -457,8 +427,7 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
 #pragma unroll
               for (int column = 0; column < 32; ++column)
                 values[column] = __uint_as_float(raw[column]);
-              finish_chunk<mode>(args, values, chunk, feature, feature_base, lane, scale,
-                                 row_best);
+              finish_chunk(args, values, chunk, feature, scale);
             }
           }
         }
@@ -469,6 +438,7 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
       if (lane == 0)
         ptx::mbarrier_arrive(acc_empty_bar + 8U * buffer);
       }
+
     }
     if constexpr (mode == 2) {
       // Every tile of this CTA is in row_best: one global atomic per row and CTA. One per tile and
@@ -776,6 +746,31 @@ int launch_mode(const LinearPlan &plan, const KernelArguments &arguments, cudaSt
                                  : launch_rows_bucket<mode, false>(plan, arguments, stream);
 }
 
+// Plain epilogues: the kernel that the plan was scheduled for.
+template <int mode>
+int launch_planned(const LinearPlan &plan, const KernelArguments &arguments, cudaStream_t stream) {
+  return plan.tile_width == pair_features ? launch_pair_linear(plan, arguments, mode, stream)
+                                          : launch_mode<mode>(plan, arguments, stream);
+}
+
+// Single CTAs or pairs. More rows than a tile holds need the pairs' row tiles. Up to 256 rows the
+// pairs pay where the activation half of a tile is what an SM has too much of, K is not cut (their
+// start and end cost two cluster barriers) and a tile is long enough to hide those: bf16
+// 5376 -> 43008 at 256 rows 103 us against 119, 192 rows 85 against 91, 128 rows 79 against 79,
+// 24 rows 70 against 68; e4m3 256 rows 59 to 64 against 67 to 73, 192 rows 54 against 54; but
+// bf16 1024 -> 262144 (16 blocks of K) 240 against 235 at 256 rows.
+bool schedule_plain(LinearPlan *plan, int rows, int input_width, int output_width,
+                    int requested_splits, int element_bytes) {
+  schedule_linear(plan, rows, input_width, output_width, requested_splits, element_bytes);
+  if (rows > 256)
+    return schedule_pairs(plan);
+  if (plan->splits == 1 && plan->tiles >= plan->ctas / 2 && plan->k_blocks >= 32 &&
+      rows > (element_bytes == 2 ? 160 : 192)) {
+    schedule_pairs(plan);   // keeps the plan when it cannot
+  }
+  return true;
+}
+
 // `split` false: one piece per tile whatever the plan says (bf16 store and argmax epilogues).
 KernelArguments base_arguments(const LinearPlan &plan, int *device_error, bool split) {
   KernelArguments arguments{};
@@ -804,13 +799,13 @@ std::size_t linear_partial_bytes_for(int rows, int input_width, int output_width
   if (rows <= 0 || rows > 256 || input_width <= 0 || output_width <= 0)
     return 0;
   LinearPlan plan{};
-  schedule_linear(&plan, rows, input_width, output_width, 0, element_bytes);
+  schedule_plain(&plan, rows, input_width, output_width, 0, element_bytes);
   return linear_partial_bytes(plan);
 }
 
 int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_weight, int rows,
                      int input_width, int output_width, int requested_splits, const char **error,
-                     int element_bytes) {
+                     int element_bytes, int most_rows) {
   const auto fail = [&](const char *message, int code) {
     if (error != nullptr)
       *error = message;
@@ -822,7 +817,7 @@ int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_we
   }
   if (element_bytes != 1 && element_bytes != 2)
     return fail("invalid FP8 linear shape", -1);
-  if (rows > 256)
+  if (rows > most_rows)
     return fail("FP8 linear supports at most 256 rows", -2);
   if (input_width * element_bytes % 16 != 0)
     return fail("FP8 linear input width must be a multiple of 16", -3);
@@ -831,12 +826,15 @@ int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_we
     return fail("FP8 linear operands must be 16-byte aligned", -4);
   }
   LinearPlan result{};
-  schedule_linear(&result, rows, input_width, output_width, requested_splits, element_bytes);
+  if (!schedule_plain(&result, rows, input_width, output_width, requested_splits, element_bytes))
+    return fail("FP8 linear cannot split this shape over CTA pairs", -6);
   const uint64_t row_bytes = static_cast<uint64_t>(input_width) * element_bytes;
+  // Each CTA, or each half of a pair, loads 128 weight rows; a pair halves the activation rows.
+  const bool pairs = result.tile_width == pair_features;
   if (!encode_byte_matrix(&result.weight_map, fp8_weight, row_bytes,
-                          static_cast<uint64_t>(output_width), tile_features) ||
+                          static_cast<uint64_t>(output_width), 128) ||
       !encode_byte_matrix(&result.input_map, fp8_input, row_bytes, static_cast<uint64_t>(rows),
-                          static_cast<uint32_t>(result.padded_rows))) {
+                          static_cast<uint32_t>(result.padded_rows / (pairs ? 2 : 1)))) {
     return fail("cuTensorMapEncodeTiled failed", -5);
   }
   *plan = result;
@@ -856,8 +854,12 @@ int make_gated_linear_plan(LinearPlan *plan, const void *fp8_input, const void *
                                       2 * gated_width, 1, error, element_bytes);
   if (status != 0)
     return status;
+  // One CTA a tile here: its grid-wide phases pair columns inside a CTA.
+  schedule_linear(&result, rows, input_width, 2 * gated_width, 1, element_bytes);
   const uint64_t row_bytes = static_cast<uint64_t>(input_width) * element_bytes;
-  if (!encode_byte_matrix(&result.weight_map, fp8_weight, row_bytes,
+  if (!encode_byte_matrix(&result.input_map, fp8_input, row_bytes, static_cast<uint64_t>(rows),
+                          static_cast<uint32_t>(result.padded_rows)) ||
+      !encode_byte_matrix(&result.weight_map, fp8_weight, row_bytes,
                           static_cast<uint64_t>(2) * gated_width, tile_features / 2)) {
     if (error != nullptr)
       *error = "cuTensorMapEncodeTiled failed";
@@ -909,7 +911,7 @@ int launch_linear_bf16(const LinearPlan &plan, const float *input_scale, const f
                                                partial, device_error, stream);
     if (status != 0)
       return status;
-    const int tail_width = plan.tail_tiles * tile_features;
+    const int tail_width = plan.tail_columns();
     const size_t elements = static_cast<size_t>(plan.rows) * tail_width;
     const int blocks = static_cast<int>((elements + 255) / 256);
     return launch_chained(finalize_tail_kernel, dim3(blocks < 1184 ? blocks : 1184), dim3(256), 0,
@@ -925,7 +927,7 @@ int launch_linear_bf16(const LinearPlan &plan, const float *input_scale, const f
     arguments.input_scale = input_scale;
     arguments.weight_scale = weight_scale;
     arguments.output = static_cast<__nv_bfloat16 *>(bf16_output);
-    return launch_mode<0>(plan, arguments, stream);
+    return launch_planned<0>(plan, arguments, stream);
   }
   const int status = launch_linear_partial(plan, partial, device_error, stream);
   if (status != 0)
@@ -953,13 +955,13 @@ int launch_linear_bf16_tail(const LinearPlan &plan, const float *input_scale,
   arguments.tail_tiles = plan.tail_tiles;
   arguments.tail_splits = plan.tail_splits;
   arguments.tail_k_blocks_per_split = plan.tail_k_blocks_per_split;
-  return launch_mode<0>(plan, arguments, stream);
+  return launch_planned<0>(plan, arguments, stream);
 }
 
 std::size_t linear_tail_bytes(const LinearPlan &plan) {
   return plan.tail_tiles <= 0 ? 0
                               : sizeof(float) * static_cast<std::size_t>(plan.tail_splits) *
-                                    plan.rows * plan.tail_tiles * tile_features;
+                                    plan.rows * plan.tail_columns();
 }
 
 int launch_linear_partial(const LinearPlan &plan, float *partial, int *device_error,
@@ -968,7 +970,7 @@ int launch_linear_partial(const LinearPlan &plan, float *partial, int *device_er
     return -13;
   KernelArguments arguments = base_arguments(plan, device_error, true);
   arguments.partial = partial;
-  return launch_mode<1>(plan, arguments, stream);
+  return launch_planned<1>(plan, arguments, stream);
 }
 
 int launch_linear_argmax(const LinearPlan &plan, const float *input_scale,
@@ -980,7 +982,7 @@ int launch_linear_argmax(const LinearPlan &plan, const float *input_scale,
   arguments.input_scale = input_scale;
   arguments.weight_scale = weight_scale;
   arguments.best = best;
-  return launch_mode<2>(plan, arguments, stream);
+  return launch_planned<2>(plan, arguments, stream);
 }
 
 int launch_unpack_best(const unsigned long long *best, int *tokens, int rows,

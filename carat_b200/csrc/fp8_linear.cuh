@@ -24,7 +24,8 @@ struct LinearPlan {
   int input_width{0};
   int output_width{0};
   int padded_rows{0};       // UMMA N: 32, 64, 128, 192 or 256
-  int tiles{0};             // output-feature tiles of 128
+  int tile_width{0};        // output features per tile: 256 (CTA pairs), 128 in a gated plan
+  int tiles{0};             // output-feature tiles
   int k_blocks{0};          // 128-byte K blocks
   int ctas{0};              // persistent CTAs (multiprocessor count)
   int splits{1};            // K pieces per tile when there are fewer tiles than SMs
@@ -34,6 +35,7 @@ struct LinearPlan {
   int tail_tiles{0};
   int tail_splits{1};
   int tail_k_blocks_per_split{0};
+  int tail_columns() const { return output_width - (tiles - tail_tiles) * tile_width; }
   int element_bytes{1};     // 1: e4m3 operands; 2: bf16 operands (scales are then ignored)
   // Gated plan (make_gated_linear_plan): the weight is [gate rows | up rows], output_width is
   // 2 * gated_width, a tile pairs 64 gate features with their 64 up features and weight_map's
@@ -47,7 +49,7 @@ struct LinearPlan {
 // the launch functions then take null scales and multiply by one.
 int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_weight, int rows,
                      int input_width, int output_width, int requested_splits, const char **error,
-                     int element_bytes = 1);
+                     int element_bytes = 1, int most_rows = 256);
 
 // The gate_up linear with GeGLU in its epilogue. `fp8_weight` is [2 * gated_width, input_width]
 // with the gate rows first; gated_width must be a multiple of 64.

@@ -37,6 +37,33 @@ inline bool pdl_enabled() {
   return enabled;
 }
 
+// The same for a grid of clusters of `cluster` CTAs.
+template <typename... KernelArgs, typename... Args>
+cudaError_t launch_clustered(void (*kernel)(KernelArgs...), dim3 grid, dim3 block,
+                             size_t shared_bytes, cudaStream_t stream, unsigned int cluster,
+                             Args... args) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = shared_bytes;
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  unsigned int count = 0;
+  attributes[count].id = cudaLaunchAttributeClusterDimension;
+  attributes[count].val.clusterDim.x = cluster;
+  attributes[count].val.clusterDim.y = 1;
+  attributes[count].val.clusterDim.z = 1;
+  ++count;
+  if (pdl_enabled()) {
+    attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[count].val.programmaticStreamSerializationAllowed = 1;
+    ++count;
+  }
+  config.attrs = attributes;
+  config.numAttrs = count;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
+}
+
 template <typename... KernelArgs, typename... Args>
 cudaError_t launch_chained(void (*kernel)(KernelArgs...), dim3 grid, dim3 block,
                            size_t shared_bytes, cudaStream_t stream, bool cooperative,

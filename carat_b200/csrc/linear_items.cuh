@@ -29,7 +29,7 @@ struct KernelArguments {
   int splits;                 // K pieces per tile (1 unless mode 1)
   int k_blocks_per_split;
   // Mode 0 only: the last `tail_tiles` feature tiles are cut into `tail_splits` K pieces whose
-  // fp32 partial sums go to tail_partial [piece, rows, tail_tiles * 128] instead of `output`.
+  // fp32 partial sums go to tail_partial [piece, rows, columns of those tiles] instead of `output`.
   float *tail_partial;
   int tail_tiles;
   int tail_splits;
@@ -108,6 +108,7 @@ inline void schedule_linear(LinearPlan *plan, int rows, int input_width, int out
   result.input_width = input_width;
   result.output_width = output_width;
   result.element_bytes = element_bytes;
+  result.tile_width = tile_features;
   result.padded_rows = rows <= 32 ? 32 : rows <= 64 ? 64 : rows <= 128 ? 128 : rows <= 192 ? 192 : 256;
   result.tiles = (output_width + tile_features - 1) / tile_features;
   result.k_blocks = (input_width * element_bytes + tile_k_elements - 1) / tile_k_elements;

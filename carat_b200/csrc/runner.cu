@@ -967,14 +967,15 @@ void verify_step(Runner &runner, const int *proposals, int requests, int depth,
       auto *partials = runner.split_partials.get<float>();
       const LinearPlan &up = plan.gate_up_int4.schedule;
       TailSource tail{};
-      if (up.splits == 1 && up.tail_tiles > 0 && up.tail_tiles * 128 <= config.intermediate_size) {
+      if (up.splits == 1 && up.tail_tiles > 0 &&
+          up.tail_columns() <= config.intermediate_size) {
         require_launch(launch_int4_linear_bf16_tail(plan.gate_up_int4, runner.gate_up.get(),
                                                     partials, runner.device_error, stream),
                        "INT4 linear");
         runner.launches += 1;
         tail = TailSource{partials, up.tail_splits,
-                          2 * config.intermediate_size - up.tail_tiles * 128, up.tail_tiles * 128,
-                          unit, unit};
+                          2 * config.intermediate_size - up.tail_columns(), up.tail_columns(), unit,
+                          unit};
       } else {
         require_launch(launch_int4_linear_bf16(plan.gate_up_int4, runner.gate_up.get(), partials,
                                                runner.device_error, stream),
@@ -1033,7 +1034,7 @@ void verify_step(Runner &runner, const int *proposals, int requests, int depth,
     TailSource tail{};
     if (plan.gate_up.tail_tiles > 0 &&
         linear_tail_bytes(plan.gate_up) <= runner.split_partials.bytes() &&
-        plan.gate_up.tail_tiles * 128 <= config.intermediate_size) {
+        plan.gate_up.tail_columns() <= config.intermediate_size) {
       require_launch(launch_linear_bf16_tail(plan.gate_up, scales + word + 2, w.gate_up_scale,
                                              runner.gate_up.get(),
                                              runner.split_partials.get<float>(),
@@ -1041,8 +1042,8 @@ void verify_step(Runner &runner, const int *proposals, int requests, int depth,
                      "FP8 linear");
       runner.launches += 1;
       tail = TailSource{runner.split_partials.get<float>(), plan.gate_up.tail_splits,
-                        2 * config.intermediate_size - plan.gate_up.tail_tiles * 128,
-                        plan.gate_up.tail_tiles * 128, scales + word + 2, w.gate_up_scale};
+                        2 * config.intermediate_size - plan.gate_up.tail_columns(),
+                        plan.gate_up.tail_columns(), scales + word + 2, w.gate_up_scale};
     } else {
       run_linear(runner, plan.gate_up, scales + word + 2, w.gate_up_scale, runner.gate_up.get(),
                  false);

@@ -1,0 +1,57 @@
+"""The linear's CTA-pair kernel (calls of many rows) against fp32 and against the single-CTA kernel.
+
+Both kernels take every sum in the same order (the K pieces and the K-cut tail depend on the widths
+only), so a row's result may not depend on how many rows its call has: bit-equal, not close.
+Against fp32 the bar is the bf16 rounding of the output, 2^-9 relative to a value, plus the
+accumulation order; 4e-3 norm-wise is twice that rounding's worst case.
+"""
+import pytest
+import torch
+
+import carat_b200
+from carat_b200.capi import check
+from helpers import rms_relative_error
+
+pytestmark = pytest.mark.gpu
+
+# (rows of the wide call, K, N): edges of the row tile, odd 128-feature tile counts, a K-cut tail,
+# a last feature tile that is half empty, K that is not a whole number of blocks.
+SHAPES = [(161, 4096, 16384), (193, 5376, 43008), (224, 4112, 19200), (256, 5376, 18944 + 128),
+          (255, 8192, 9472 + 64)]
+
+
+@pytest.mark.parametrize("wide", [False, True], ids=["e4m3", "bf16"])
+@pytest.mark.parametrize("rows,k,n", SHAPES)
+def test_rows_do_not_depend_on_the_call_they_are_in(cuda_device, wide, rows, k, n):
+    library = carat_b200.library()
+    generator = torch.Generator(device="cuda").manual_seed(rows + n)
+    x = torch.randn(rows, k, device="cuda", generator=generator).to(torch.bfloat16)
+    w = (torch.randn(n, k, device="cuda", generator=generator) * 0.02).to(torch.bfloat16)
+    if not wide:
+        x, x_scale = carat_b200.quantize_tensor_to_fp8(x)
+        w, w_scale = carat_b200.quantize_tensor_to_fp8(w)
+
+    def linear(count):
+        out = torch.full((count, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+        size = (library.carat_b200_bf16_linear_workspace_bytes if wide
+                else library.carat_b200_fp8_linear_workspace_bytes)(count, k, n)
+        workspace = torch.empty(max(size, 16), dtype=torch.uint8, device="cuda")
+        if wide:
+            check(library.carat_b200_bf16_linear(x.data_ptr(), w.data_ptr(), out.data_ptr(), count,
+                                                 k, n, workspace.data_ptr(), size, None))
+        else:
+            check(library.carat_b200_fp8_linear(
+                x.data_ptr(), x_scale.data_ptr(), w.data_ptr(), w_scale.data_ptr(),
+                out.data_ptr(), count, k, n, workspace.data_ptr(), size, None))
+        torch.cuda.synchronize()
+        return out
+
+    many = linear(rows)
+    few = linear(100)
+    assert torch.equal(many[:100].view(torch.int16), few.view(torch.int16))
+    if wide:
+        want = x.float() @ w.float().t()
+    else:
+        want = ((x.view(torch.float8_e4m3fn).float() @ w.view(torch.float8_e4m3fn).float().t())
+                * (x_scale * w_scale))
+    assert rms_relative_error(many, want) < 4e-3
