@@ -10,7 +10,7 @@ import subprocess
 import sys
 
 PACKAGE = os.path.dirname(os.path.abspath(__file__))
-SOURCES = ["fp8_linear.cu", "fp8_linear_static.cu", "pair_linear.cu", "int4_linear.cu", "row_ops.cu", "qkv_post.cu", "attention_simt.cu", "attention_tc.cu",
+SOURCES = ["fp8_linear.cu", "fp8_linear_static.cu", "pair_linear.cu", "prefill_attention.cu", "int4_linear.cu", "row_ops.cu", "qkv_post.cu", "attention_simt.cu", "attention_tc.cu",
     "attention_fused.cu", "attention_stream.cu", "accept.cu",
            "context.cu", "selftest.cu", "weights.cu", "placement.cu", "runner.cu", "capi_linear.cu", "capi_ops.cu"]
 LIBRARY = os.path.join(PACKAGE, "libcarat_b200.so")

@@ -841,6 +841,25 @@ int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_we
   return 0;
 }
 
+int retarget_linear_plan(LinearPlan *plan, const void *input, int rows) {
+  LinearPlan result{};
+  result.weight_map = plan->weight_map;
+  if (rows <= 0 || (reinterpret_cast<uintptr_t>(input) & 15U) != 0 ||
+      !schedule_plain(&result, rows, plan->input_width, plan->output_width, 0,
+                      plan->element_bytes)) {
+    return -1;
+  }
+  const bool pairs = result.tile_width == pair_features;
+  if (!encode_byte_matrix(&result.input_map, input,
+                          static_cast<uint64_t>(plan->input_width) * plan->element_bytes,
+                          static_cast<uint64_t>(rows),
+                          static_cast<uint32_t>(result.padded_rows / (pairs ? 2 : 1)))) {
+    return -5;
+  }
+  *plan = result;
+  return 0;
+}
+
 int make_gated_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_weight,
                            int rows, int input_width, int gated_width, const char **error,
                            int element_bytes) {

@@ -51,6 +51,10 @@ int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_we
                      int input_width, int output_width, int requested_splits, const char **error,
                      int element_bytes = 1, int most_rows = 256);
 
+// The same plan for another number of rows of another input of the same width: the schedule and
+// the input map are made again, the weight map stays.
+int retarget_linear_plan(LinearPlan *plan, const void *input, int rows);
+
 // The gate_up linear with GeGLU in its epilogue. `fp8_weight` is [2 * gated_width, input_width]
 // with the gate rows first; gated_width must be a multiple of 64.
 int make_gated_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_weight,

@@ -4,7 +4,7 @@
 //   output[rows, N] = bf16( scale * X[rows, K] . W[N, K]^T ), fp32 accumulation.
 //
 // Up to 256 rows the problem is HBM-bound, so it is a weight stream with swapped operands: output
-// features are the UMMA M dimension, activation rows (padded to 32) its N dimension. Two SMs work
+// features are the UMMA M dimension, activation rows (padded to 16 or 32) its N dimension. Two SMs work
 // on one tile of 256 features: each CTA of a pair streams its own 128 weight rows and HALF of the
 // activation rows, and one tcgen05.mma of the pair (M = 256) reads both halves. Against one CTA
 // per 128 features that halves the activation bytes each SM fetches from L2, writes to shared
@@ -421,7 +421,7 @@ pair_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
 template <int mode, bool wide>
 int launch_pairs(const LinearPlan &plan, const KernelArguments &arguments, cudaStream_t stream) {
   PairShape shape{};
-  shape.tile_rows = pair_tile_rows(plan.rows);
+  shape.tile_rows = pair_tile_rows(plan.rows, plan.element_bytes);
   shape.row_tiles = pair_row_tiles(plan.rows);
   if (mode == 2 && shape.row_tiles > 1)
     return -12;
@@ -458,7 +458,7 @@ bool schedule_pairs(LinearPlan *plan) {
   if ((result.tiles - result.tail_tiles) % 2 != 0 && result.tail_tiles > 0)
     return false;
   result.tile_width = pair_features;
-  result.padded_rows = pair_tile_rows(result.rows);
+  result.padded_rows = pair_tile_rows(result.rows, result.element_bytes);
   result.tiles = (result.tiles + 1) / 2;
   result.tail_tiles = (result.tail_tiles + 1) / 2;
   return true;

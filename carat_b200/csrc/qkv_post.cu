@@ -224,6 +224,92 @@ template <int per> __global__ void qkv_post_kernel(QkvPostArguments a) {
                     value_high);
 }
 
+template <int per> __global__ void prefill_qkv_post_kernel(PrefillQkvArguments a) {
+  constexpr int dimension = per * 64;
+  grid_dependency_launch();
+  const int warp = static_cast<int>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x / 32);
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const int heads_per_row = a.query_heads + a.kv_heads;
+  if (warp >= a.rows * heads_per_row)
+    return;
+  const int row = warp / heads_per_row;
+  const int head = warp % heads_per_row;
+  const bool is_query = head < a.query_heads;
+  const int kv_head = head - a.query_heads;
+  const int query_width = a.query_heads * dimension;
+  const int kv_width = a.kv_heads * dimension;
+  const int packed_width = query_width + kv_width * (a.key_equals_value ? 1 : 2);
+  // Norm weights, positions and cos/sin rows are inputs of the step: fetched before the wait.
+  RopeOperands<per> with;
+  load_halves<per>(static_cast<const __nv_bfloat16 *>(is_query ? a.query_norm : a.key_norm), lane,
+                   with.weight_low, with.weight_high);
+  const int position = a.positions[row];
+  if (position < 0 || position >= a.max_positions)
+    return;
+  const size_t table_row = static_cast<size_t>(position) * dimension;
+  load_halves<per>(static_cast<const __nv_bfloat16 *>(a.cosine) + table_row, lane, with.cosine_low,
+                   with.cosine_high);
+  load_halves<per>(static_cast<const __nv_bfloat16 *>(a.sine) + table_row, lane, with.sine_low,
+                   with.sine_high);
+  grid_dependency_wait();
+
+  const auto *packed_row =
+      static_cast<const __nv_bfloat16 *>(a.packed) + static_cast<size_t>(row) * packed_width;
+  float low[per];
+  float high[per];
+  float value_low[per];
+  float value_high[per];
+  load_halves<per>(packed_row + (is_query ? head * dimension : query_width + kv_head * dimension),
+                   lane, low, high);
+  const bool separate_value = !is_query && !a.key_equals_value;
+  if (separate_value)
+    load_halves<per>(packed_row + query_width + kv_width + kv_head * dimension, lane, value_low,
+                     value_high);
+  const float inverse_rms = inverse_rms_of<per>(low, high, a.epsilon);
+  float out_low[per];
+  float out_high[per];
+  norm_rope<per>(low, high, inverse_rms, with, out_low, out_high);
+  if (is_query) {
+    store_halves<per>(static_cast<__nv_bfloat16 *>(a.queries) +
+                          static_cast<size_t>(row) * query_width + head * dimension,
+                      lane, out_low, out_high);
+    return;
+  }
+  float inverse_value_rms = inverse_rms;
+  if (separate_value) {
+    inverse_value_rms = inverse_rms_of<per>(value_low, value_high, a.epsilon);
+  } else {
+#pragma unroll
+    for (int index = 0; index < per; ++index) {
+      value_low[index] = low[index];
+      value_high[index] = high[index];
+    }
+  }
+#pragma unroll
+  for (int index = 0; index < per; ++index) {
+    value_low[index] *= inverse_value_rms;
+    value_high[index] *= inverse_value_rms;
+  }
+  if (a.staged_rows != nullptr) {
+    const size_t destination =
+        static_cast<size_t>(a.staged_rows[row]) * kv_width + kv_head * dimension;
+    store_halves<per>(static_cast<__nv_bfloat16 *>(a.staged_keys) + destination, lane, out_low,
+                      out_high);
+    store_halves<per>(static_cast<__nv_bfloat16 *>(a.staged_values) + destination, lane, value_low,
+                      value_high);
+  }
+  const int slot = a.cache_slots[row];
+  if (slot >= 0) {
+    const size_t destination =
+        static_cast<size_t>(slot * a.slot_stride + kv_head * a.head_stride) +
+        static_cast<size_t>(position % a.capacity) * dimension;
+    store_halves<per>(static_cast<__nv_bfloat16 *>(a.key_cache) + destination, lane, out_low,
+                      out_high);
+    store_halves<per>(static_cast<__nv_bfloat16 *>(a.value_cache) + destination, lane, value_low,
+                      value_high);
+  }
+}
+
 template <int per>
 __global__ void query_post_kernel(const __nv_bfloat16 *projected, const __nv_bfloat16 *weight,
                                   const __nv_bfloat16 *cosine_table,
@@ -307,6 +393,32 @@ int launch_qkv_post(const QkvPostArguments &a, cudaStream_t stream) {
     break;
   case 512:
     launch_chained(qkv_post_kernel<8>, dim3(blocks), dim3(128), 0, stream, false, a);
+    break;
+  default:
+    return -3;
+  }
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : -11;
+}
+
+int launch_prefill_qkv_post(const PrefillQkvArguments &a, cudaStream_t stream) {
+  if (a.packed == nullptr || a.query_norm == nullptr || a.key_norm == nullptr ||
+      a.cosine == nullptr || a.sine == nullptr || a.queries == nullptr || a.positions == nullptr ||
+      a.cache_slots == nullptr || a.key_cache == nullptr || a.value_cache == nullptr ||
+      (a.staged_rows != nullptr && (a.staged_keys == nullptr || a.staged_values == nullptr)) ||
+      a.rows <= 0 || a.query_heads <= 0 || a.kv_heads <= 0 || a.capacity <= 0 ||
+      a.slot_stride % 8 != 0 || a.head_stride % 8 != 0 ||
+      !aligned16(a.packed, a.query_norm, a.key_norm, a.cosine, a.sine, a.queries, a.key_cache,
+                 a.value_cache, a.staged_keys, a.staged_values)) {
+    return -1;
+  }
+  const int warps = a.rows * (a.query_heads + a.kv_heads);
+  const int blocks = (warps + 3) / 4;
+  switch (a.head_dim) {
+  case 256:
+    launch_chained(prefill_qkv_post_kernel<4>, dim3(blocks), dim3(128), 0, stream, false, a);
+    break;
+  case 512:
+    launch_chained(prefill_qkv_post_kernel<8>, dim3(blocks), dim3(128), 0, stream, false, a);
     break;
   default:
     return -3;

@@ -47,6 +47,38 @@ struct QkvPostArguments {
 
 int launch_qkv_post(const QkvPostArguments &arguments, cudaStream_t stream);
 
+// The same for a prefill step: packed rows of several requests, position and owner per row.
+// Q goes to [rows, query_heads, head_dim]. A row's K and V go to the staging buffer
+// [staging rows][kv_heads * head_dim] when staged_rows is given (sliding layers), and to its slot's
+// cache at position % capacity when cache_slots[row] >= 0.
+struct PrefillQkvArguments {
+  const void *packed;
+  const void *query_norm;
+  const void *key_norm;
+  const void *cosine;
+  const void *sine;
+  void *queries;
+  const int *positions;        // [rows]
+  const int *cache_slots;      // [rows]
+  const int *staged_rows;      // [rows], may be null
+  void *staged_keys;
+  void *staged_values;
+  void *key_cache;
+  void *value_cache;
+  long long slot_stride;       // elements
+  long long head_stride;
+  int rows;
+  int capacity;
+  int query_heads;
+  int kv_heads;
+  int head_dim;                // 256 or 512
+  int key_equals_value;
+  int max_positions;
+  float epsilon;
+};
+
+int launch_prefill_qkv_post(const PrefillQkvArguments &arguments, cudaStream_t stream);
+
 // Query-only variant for the drafter (cuda/qkv.cu run_query_ragged): one row per request,
 // rotated at positions[r] + position_offset. Output [requests, query_heads, 1, head_dim].
 // inputs_static: as in QkvPostArguments.

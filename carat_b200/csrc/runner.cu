@@ -12,6 +12,7 @@
 #include "context.cuh"
 #include "fp8_linear.cuh"
 #include "int4_linear.cuh"
+#include "prefill_attention.cuh"
 #include "qkv_post.cuh"
 #include "row_ops.cuh"
 
@@ -29,6 +30,9 @@ namespace {
 
 constexpr int maximum_depth = 9;       // k = 8 drafts + the forced token
 constexpr int prefill_pieces = 64;     // (slot, eight-token piece) entries one prefill step takes
+// Rows of a packed BF16 prefill step (prefill_rows_step). At 2048 rows the linears are bound by
+// the tensor cores (0.9 us a row and 31B layer against 154 us to stream its weights).
+constexpr int packed_prefill_rows = 2048;
 constexpr int maximum_rows = 256;      // rows one FP8 linear launch accepts (24 slots x depth 9 = 216)
 constexpr int global_chunk_keys = 1024;
 
@@ -219,6 +223,19 @@ struct carat_b200_runner {
   // so their per-request inputs are sized for prefill_pieces entries, not for the batch.
   DeviceBuffer p_step_inputs, p_request_chunks;
   PinnedBuffer p_host_inputs;
+  // Packed prefill steps: row buffers for packed_prefill_rows rows, the staging region of the
+  // sliding layers (one layer at a time), per-row and per-tile inputs, and the layers' weight maps.
+  struct PrefillLayer {
+    LinearPlan qkv, o, gate_up, down;   // only their weight maps are used
+  };
+  std::vector<PrefillLayer> q_layers;
+  DeviceBuffer q_hidden_a, q_hidden_b, q_residual, q_normed, q_pre_mlp, q_activated, q_packed,
+      q_queries, q_attention, q_projected, q_gate_up, q_final, q_partials, q_staged, q_inputs,
+      q_last_rows;
+  PinnedBuffer q_host_inputs;
+  size_t q_staged_value_offset{0};
+  int q_staging_rows{0};
+  bool packed_prefill{false};
   std::map<std::pair<int, int>, AttentionMaps> direct_maps;   // sliding layers read as linear caches
   std::map<int, StepPlans> prefill_plans;
   // ---- drafter precision (CARAT_B200_ASSISTANT_FP8_*): bf16 matrices and their plans
@@ -577,10 +594,10 @@ StepPlans &draft_plans_for(Runner &runner, int rows) {
 }
 
 LinearPlan plan_bf16_linear(const void *input, const void *weight, int rows, int in, int out,
-                            int splits) {
+                            int splits, int most_rows = maximum_rows) {
   LinearPlan plan;
   const char *message = "invalid BF16 linear shape";
-  if (make_linear_plan(&plan, input, weight, rows, in, out, splits, &message, 2) != 0)
+  if (make_linear_plan(&plan, input, weight, rows, in, out, splits, &message, 2, most_rows) != 0)
     throw Failure{"invalid BF16 linear shape"};
   return plan;
 }
@@ -1403,6 +1420,464 @@ void prefill_step(Runner &runner, const int *tokens, int requests, int depth, co
   runner.last_rows = rows;
 }
 
+// Where the pieces of a packed prefill step's input block are, in ints.
+struct PackedInputs {
+  int tokens, positions, sliding_slots, global_slots, staged_rows, last_rows, last_slots;
+  int segments, tiles, total;
+  PackedInputs(int rows, int batch, int most_tiles) {
+    int at = 0;
+    const auto take = [&](int count) {
+      const int here = at;
+      at += (count + 3) / 4 * 4;
+      return here;
+    };
+    tokens = take(rows);
+    positions = take(rows);
+    sliding_slots = take(rows);
+    global_slots = take(rows);
+    staged_rows = take(rows);
+    last_rows = take(batch);
+    last_slots = take(batch);
+    segments = take(batch * static_cast<int>(sizeof(PrefillSegment) / sizeof(int)));
+    tiles = take(most_tiles * static_cast<int>(sizeof(PrefillTile) / sizeof(int)));
+    total = at;
+  }
+};
+
+// Most query tiles of a step over all the tile sizes its layers use: a segment ends with a partial
+// tile, and a tile holds at least one row.
+int packed_prefill_tiles(const Runner &runner) {
+  int most = 0;
+  for (const LayerState &layer : runner.layers) {
+    const int tokens = 128 / (layer.shape.query_heads / layer.shape.kv_heads);
+    most += packed_prefill_rows / tokens + runner.batch;
+  }
+  // One list per distinct tile size; layers share them.
+  return std::min(most, 8 * (packed_prefill_rows + runner.batch));
+}
+
+bool packed_prefill_takes(const Runner &runner) {
+  for (const LayerState &layer : runner.layers) {
+    if (!prefill_attention_takes(layer.shape.query_heads, layer.shape.kv_heads,
+                                 layer.shape.head_dim))
+      return false;
+  }
+  return runner.config.hidden_size % 8 == 0;
+}
+
+// Rows of a segment's staging region: from the tile that holds the oldest visible position to the
+// end of the tile that holds its last row.
+PrefillSegment packed_segment(const Runner &runner, int slot, int first, int count) {
+  const int window = runner.config.sliding_window;
+  const int lowest = first >= window ? first - window + 1 : 0;
+  PrefillSegment segment{};
+  segment.slot = slot;
+  segment.first = first;
+  segment.count = count;
+  segment.origin = lowest / prefill_key_tile * prefill_key_tile;
+  segment.stage_rows = (first + count - segment.origin + prefill_key_tile - 1) /
+                       prefill_key_tile * prefill_key_tile;
+  return segment;
+}
+
+void prepare_packed_prefill(Runner &runner) {
+  const auto &config = runner.config;
+  const size_t rows = packed_prefill_rows;
+  const size_t row_hidden = rows * config.hidden_size * 2;
+  size_t widest_query = 0;
+  size_t widest_packed = 0;
+  size_t widest_staged = 0;
+  for (const LayerState &layer : runner.layers) {
+    widest_query = std::max(widest_query, static_cast<size_t>(layer.query_width()));
+    widest_packed = std::max(widest_packed, static_cast<size_t>(layer.packed_width()));
+    if (!layer.shape.global_attention)
+      widest_staged = std::max(widest_staged, static_cast<size_t>(layer.kv_width()));
+  }
+  for (DeviceBuffer *buffer : {&runner.q_hidden_a, &runner.q_hidden_b, &runner.q_residual,
+                               &runner.q_normed, &runner.q_pre_mlp, &runner.q_projected,
+                               &runner.q_final})
+    buffer->allocate(row_hidden);
+  runner.q_activated.allocate(rows * config.intermediate_size * 2);
+  runner.q_packed.allocate(rows * widest_packed * 2);
+  runner.q_queries.allocate(rows * widest_query * 2, true);
+  runner.q_attention.allocate(rows * widest_query * 2);
+  runner.q_gate_up.allocate(rows * 2 * config.intermediate_size * 2);
+  runner.q_last_rows.allocate(static_cast<size_t>(runner.batch) * config.hidden_size * 2);
+  // Every segment brings at most a window and two partial tiles beside its own rows.
+  const int window_rows = std::min(config.sliding_window, runner.maximum_context);
+  runner.q_staging_rows =
+      packed_prefill_rows + runner.batch * (window_rows + 2 * prefill_key_tile);
+  runner.q_staged_value_offset = align_up(runner.q_staging_rows * widest_staged * 2);
+  if (widest_staged > 0)
+    runner.q_staged.allocate(2 * runner.q_staged_value_offset, true);
+  const PackedInputs layout(packed_prefill_rows, runner.batch, packed_prefill_tiles(runner));
+  runner.q_inputs.allocate(sizeof(int) * static_cast<size_t>(layout.total), true);
+  runner.q_host_inputs.allocate(sizeof(int) * static_cast<size_t>(layout.total));
+  if (runner.unit_scale.get() == nullptr) {
+    const float one = 1.0F;
+    runner.unit_scale.allocate(sizeof(float));
+    require_cuda(cudaMemcpy(runner.unit_scale.get(), &one, sizeof(float), cudaMemcpyHostToDevice),
+                 "set unit scale");
+  }
+  size_t partial_bytes = 0;
+  runner.q_layers.clear();
+  for (size_t index = 0; index < runner.layers.size(); ++index) {
+    const LayerState &layer = runner.layers[index];
+    const carat_b200_layer_bf16_weights &weights = runner.bf16_layers[index];
+    const auto plan = [&](const void *input, const void *weight, int in, int out) {
+      const LinearPlan made = plan_bf16_linear(input, weight, packed_prefill_rows, in, out, 0,
+                                               packed_prefill_rows);
+      partial_bytes = std::max(partial_bytes, linear_partial_bytes(made));
+      return made;
+    };
+    Runner::PrefillLayer entry;
+    entry.qkv = plan(runner.q_normed.get(), weights.qkv, config.hidden_size, layer.packed_width());
+    entry.o = plan(runner.q_attention.get(), weights.o, layer.query_width(), config.hidden_size);
+    entry.gate_up = plan(runner.q_pre_mlp.get(), weights.gate_up, config.hidden_size,
+                         2 * config.intermediate_size);
+    entry.down = plan(runner.q_activated.get(), weights.down, config.intermediate_size,
+                      config.hidden_size);
+    runner.q_layers.push_back(entry);
+  }
+  runner.q_partials.allocate(std::max<size_t>(partial_bytes, 256));
+}
+
+// One BF16 forward over consecutive prompt rows of several slots, all of them made resident: the
+// rows of segment s are tokens[offset of s ..], positions first .. first + count - 1 of its slot.
+// Rows of different segments only share the linears, and every sum's order depends on the widths
+// and on a row's position alone, so a row's result does not depend on the step it is in.
+// `complete[s]` marks segments whose last row ends a prompt: its final-normed hidden row goes to the
+// slot's hand-off row and the bf16 LM head predicts its next token into predictions[s].
+void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
+                       std::vector<PrefillSegment> &segments, const std::vector<bool> &complete,
+                       std::vector<int> &predictions) {
+  const auto &config = runner.config;
+  const int rows = static_cast<int>(tokens.size());
+  const int hidden = config.hidden_size;
+  const float epsilon = config.rms_norm_epsilon;
+  const int most_tiles = packed_prefill_tiles(runner);
+  const PackedInputs layout(packed_prefill_rows, runner.batch, most_tiles);
+  int *host = runner.q_host_inputs.get<int>();
+  const int *device = runner.q_inputs.get<int>();
+  cudaStream_t stream = runner.stream;
+  const int sliding_capacity = std::min(runner.maximum_context, config.sliding_window);
+
+  // ---- per-row inputs, staging regions, query tiles
+  int row = 0;
+  int stage_row = 0;
+  int last_count = 0;
+  for (size_t index = 0; index < segments.size(); ++index) {
+    PrefillSegment &segment = segments[index];
+    segment.stage_row = stage_row;
+    stage_row += segment.stage_rows;
+    for (int token = 0; token < segment.count; ++token, ++row) {
+      const int position = segment.first + token;
+      host[layout.tokens + row] = tokens[static_cast<size_t>(row)];
+      host[layout.positions + row] = position;
+      // Of a long segment only the rows the ring keeps may be written: earlier ones share theirs.
+      host[layout.sliding_slots + row] =
+          token >= segment.count - sliding_capacity ? segment.slot : -1;
+      host[layout.global_slots + row] = segment.slot;
+      host[layout.staged_rows + row] = segment.stage_row + position - segment.origin;
+    }
+    if (complete[index]) {
+      host[layout.last_rows + last_count] = row - 1;
+      host[layout.last_slots + last_count] = segment.slot;
+      ++last_count;
+    }
+  }
+  if (rows <= 0 || rows > packed_prefill_rows || row != rows || stage_row > runner.q_staging_rows)
+    throw Failure{"invalid batched chunk prefill shape"};
+  std::memcpy(host + layout.segments, segments.data(), segments.size() * sizeof(PrefillSegment));
+  // Query tiles of every layer kind, longest key range first: the last CTAs to start then have the
+  // least to do.
+  struct TileList {
+    int tokens;
+    bool global;
+    int capacity;   // global only: rows per (slot, head) and heads, which key_base is made of
+    int heads;
+    int begin;
+    int count;
+  };
+  std::vector<TileList> lists;
+  auto *host_tiles = reinterpret_cast<PrefillTile *>(host + layout.tiles);
+  int tile_count = 0;
+  const auto tiles_for = [&](const LayerState &layer) -> const TileList & {
+    const int per_tile = 128 / (layer.shape.query_heads / layer.shape.kv_heads);
+    const bool global = layer.shape.global_attention != 0;
+    const int heads = layer.shape.kv_heads;
+    for (const TileList &list : lists) {
+      if (list.tokens == per_tile && list.global == global &&
+          (!global || (list.capacity == layer.capacity && list.heads == heads)))
+        return list;
+    }
+    TileList list{per_tile, global, layer.capacity, heads, tile_count, 0};
+    int first_row = 0;
+    for (const PrefillSegment &segment : segments) {
+      for (int token = 0; token < segment.count; token += per_tile) {
+        if (tile_count >= most_tiles)
+          throw Failure{"invalid batched chunk prefill shape"};
+        PrefillTile &tile = host_tiles[tile_count++];
+        tile.row = first_row + token;
+        tile.tokens = std::min(per_tile, segment.count - token);
+        tile.position = segment.first + token;
+        tile.key_base = global ? segment.slot * heads * layer.capacity
+                               : segment.stage_row - segment.origin;
+      }
+      first_row += segment.count;
+    }
+    list.count = tile_count - list.begin;
+    const int window = global ? 0 : config.sliding_window;
+    const auto key_rows = [window](const PrefillTile &tile) {
+      const int last = tile.position + tile.tokens;
+      return window > 0 ? std::min(last, window + tile.tokens) : last;
+    };
+    std::stable_sort(host_tiles + list.begin, host_tiles + tile_count,
+                     [&](const PrefillTile &a, const PrefillTile &b) {
+                       return key_rows(a) > key_rows(b);
+                     });
+    lists.push_back(list);
+    return lists.back();
+  };
+  std::vector<TileList> layer_tiles;
+  for (const LayerState &layer : runner.layers)
+    layer_tiles.push_back(tiles_for(layer));
+  require_cuda(cudaMemcpyAsync(runner.q_inputs.get(), host,
+                               sizeof(int) * static_cast<size_t>(layout.tiles) +
+                                   sizeof(PrefillTile) * static_cast<size_t>(tile_count),
+                               cudaMemcpyHostToDevice, stream),
+               "copy prefill step inputs");
+  auto *best = reinterpret_cast<unsigned long long *>(runner.scratch_words.get<unsigned int>() +
+                                                      runner.amax_words);
+  if (last_count > 0)
+    require_cuda(cudaMemsetAsync(best, 0, sizeof(unsigned long long) * maximum_rows, stream),
+                 "clear argmax keys");
+  require_cuda(cudaEventRecord(runner.start_event, stream), "record prefill start");
+  runner.launches = 0;
+
+  // ---- plans: schedules and input maps depend on the widths and the row count only, so layers
+  // share them and bring their weight maps.
+  std::vector<std::pair<const void *, LinearPlan>> shared;
+  const auto plan_for = [&](const LinearPlan &layer_plan, const void *input) {
+    for (const auto &entry : shared) {
+      if (entry.first == input && entry.second.input_width == layer_plan.input_width &&
+          entry.second.output_width == layer_plan.output_width) {
+        LinearPlan plan = entry.second;
+        plan.weight_map = layer_plan.weight_map;
+        return plan;
+      }
+    }
+    LinearPlan plan = layer_plan;
+    if (retarget_linear_plan(&plan, input, rows) != 0)
+      throw Failure{"invalid BF16 linear shape"};
+    shared.emplace_back(input, plan);
+    return plan;
+  };
+  auto *partials = runner.q_partials.get<float>();
+  const auto linear = [&](const LinearPlan &plan, void *output) -> PartialSource {
+    if (plan.splits > 1) {
+      require_launch(launch_linear_partial(plan, partials, runner.device_error, stream),
+                     "BF16 linear");
+      runner.launches += 1;
+      return PartialSource{partials, plan.splits, nullptr, nullptr};
+    }
+    require_launch(launch_linear_bf16(plan, nullptr, nullptr, output, partials,
+                                      runner.device_error, stream),
+                   "BF16 linear");
+    runner.launches += plan.tail_tiles > 0 ? 2 : 1;
+    return PartialSource{nullptr, 0, nullptr, nullptr};
+  };
+  const auto rows_only = [](void *rows_out) {
+    return QuantTarget{nullptr, nullptr, nullptr, nullptr, rows_out};
+  };
+
+  void *current = runner.q_hidden_a.get();
+  void *other = runner.q_hidden_b.get();
+  require_launch(launch_embed_norm_quant(runner.weights.token_embedding, device + layout.tokens,
+                                         config.vocabulary_size, runner.layers[0].weights.input_norm,
+                                         current, rows_only(runner.q_normed.get()), rows, hidden,
+                                         epsilon, nullptr, 0, stream),
+                 "embedding and input norm");
+  runner.launches += 1;
+  for (int index = 0; index < config.layer_count; ++index) {
+    const LayerState &layer = runner.layers[static_cast<size_t>(index)];
+    const Runner::PrefillLayer &plans = runner.q_layers[static_cast<size_t>(index)];
+    const auto &shape = layer.shape;
+    const auto &w = layer.weights;
+    const RopeTable &rope = *runner.rope_tables[static_cast<size_t>(layer.rope)];
+    const bool global = shape.global_attention != 0;
+    const LinearPlan qkv = plan_for(plans.qkv, runner.q_normed.get());
+    const PartialSource packed = linear(qkv, runner.q_packed.get());
+    if (packed.splits > 0) {
+      // Few output features: the K pieces are summed to bf16 rows for the post-processing.
+      require_launch(launch_quant(nullptr, partials, packed.splits, nullptr, 1,
+                                  rows_only(runner.q_packed.get()), rows, layer.packed_width(),
+                                  stream),
+                     "QKV rows");
+      runner.launches += 1;
+    }
+    void *staged_keys = runner.q_staged.get();
+    void *staged_values = runner.q_staged.get<unsigned char>() + runner.q_staged_value_offset;
+    if (!global) {
+      PrefillGatherArguments gather{};
+      gather.segments = reinterpret_cast<const PrefillSegment *>(device + layout.segments);
+      gather.segment_count = static_cast<int>(segments.size());
+      gather.key_cache = layer.keys();
+      gather.value_cache = layer.values();
+      gather.staged_keys = staged_keys;
+      gather.staged_values = staged_values;
+      gather.slot_stride = layer.slot_stride;
+      gather.head_stride = layer.head_stride;
+      gather.capacity = layer.capacity;
+      gather.window = config.sliding_window;
+      gather.kv_heads = shape.kv_heads;
+      gather.head_dim = shape.head_dim;
+      require_launch(launch_prefill_gather(gather, stream), "prefill ring rows");
+      runner.launches += 1;
+    }
+    PrefillQkvArguments post{};
+    post.packed = runner.q_packed.get();
+    post.query_norm = w.q_norm;
+    post.key_norm = w.k_norm;
+    post.cosine = rope.cosine.get();
+    post.sine = rope.sine.get();
+    post.queries = runner.q_queries.get();
+    post.positions = device + layout.positions;
+    post.cache_slots = device + (global ? layout.global_slots : layout.sliding_slots);
+    post.staged_rows = global ? nullptr : device + layout.staged_rows;
+    post.staged_keys = global ? nullptr : staged_keys;
+    post.staged_values = global ? nullptr : staged_values;
+    post.key_cache = layer.keys();
+    post.value_cache = layer.values();
+    post.slot_stride = layer.slot_stride;
+    post.head_stride = layer.head_stride;
+    post.rows = rows;
+    post.capacity = layer.capacity;
+    post.query_heads = shape.query_heads;
+    post.kv_heads = shape.kv_heads;
+    post.head_dim = shape.head_dim;
+    post.key_equals_value = shape.key_equals_value;
+    post.max_positions = runner.maximum_context;
+    post.epsilon = epsilon;
+    require_launch(launch_prefill_qkv_post(post, stream), "QKV post-processing");
+    runner.launches += 1;
+
+    const TileList &list = layer_tiles[static_cast<size_t>(index)];
+    PrefillAttentionMaps maps;
+    const int status = make_prefill_attention_maps(
+        &maps, runner.q_queries.get(), packed_prefill_rows, shape.query_heads, shape.kv_heads,
+        shape.head_dim, global ? layer.keys() : staged_keys,
+        global ? layer.values() : staged_values,
+        global ? static_cast<long long>(runner.batch) * shape.kv_heads * layer.capacity
+               : runner.q_staging_rows,
+        global ? shape.head_dim : layer.kv_width());
+    if (status != 0)
+      throw Failure{"attention tensor map encoding failed"};
+    PrefillAttentionArguments attention{};
+    attention.tiles =
+        reinterpret_cast<const PrefillTile *>(device + layout.tiles) + list.begin;
+    attention.tile_count = list.count;
+    attention.query_heads = shape.query_heads;
+    attention.kv_heads = shape.kv_heads;
+    attention.head_dim = shape.head_dim;
+    attention.window = global ? 0 : config.sliding_window;
+    attention.key_head_columns = global ? 0 : shape.head_dim;
+    attention.key_head_rows = global ? layer.capacity : 0;
+    attention.output = runner.q_attention.get();
+    attention.device_error = runner.device_error;
+    require_launch(launch_prefill_attention(maps, attention, stream), "prefill attention");
+    runner.launches += 1;
+
+    const PartialSource o_source =
+        linear(plan_for(plans.o, runner.q_attention.get()), runner.q_projected.get());
+    require_launch(launch_post_attention_norms_quant(
+                       runner.q_projected.get(), o_source, w.post_attention_norm, current,
+                       w.pre_mlp_norm, runner.q_residual.get(), rows_only(runner.q_pre_mlp.get()),
+                       rows, hidden, epsilon, stream),
+                   "post-attention norms");
+    runner.launches += 1;
+    const LinearPlan gate_up = plan_for(plans.gate_up, runner.q_pre_mlp.get());
+    TailSource tail{};
+    if (gate_up.splits == 1 && gate_up.tail_tiles > 0 &&
+        gate_up.tail_columns() <= config.intermediate_size) {
+      const float *unit = runner.unit_scale.get<float>();
+      require_launch(launch_linear_bf16_tail(gate_up, nullptr, nullptr, runner.q_gate_up.get(),
+                                             partials, runner.device_error, stream),
+                     "BF16 linear");
+      runner.launches += 1;
+      tail = TailSource{partials, gate_up.tail_splits,
+                        2 * config.intermediate_size - gate_up.tail_columns(),
+                        gate_up.tail_columns(), unit, unit};
+    } else {
+      const PartialSource up = linear(gate_up, runner.q_gate_up.get());
+      if (up.splits > 0) {
+        require_launch(launch_quant(nullptr, partials, up.splits, nullptr, 1,
+                                    rows_only(runner.q_gate_up.get()), rows,
+                                    2 * config.intermediate_size, stream),
+                       "gate_up rows");
+        runner.launches += 1;
+      }
+    }
+    require_launch(launch_geglu_quant(runner.q_gate_up.get(), tail,
+                                      rows_only(runner.q_activated.get()), rows,
+                                      config.intermediate_size, stream),
+                   "GeGLU");
+    runner.launches += 1;
+    const PartialSource down_source =
+        linear(plan_for(plans.down, runner.q_activated.get()), runner.q_projected.get());
+    const bool last = index + 1 == config.layer_count;
+    const void *next_norm = last ? runner.weights.final_norm
+                                 : runner.layers[static_cast<size_t>(index) + 1].weights.input_norm;
+    require_launch(launch_layer_output_norm_quant(
+                       runner.q_projected.get(), down_source, w.post_mlp_norm,
+                       runner.q_residual.get(), w.scalar, other, next_norm,
+                       last ? runner.q_final.get() : runner.q_normed.get(), QuantTarget{}, rows,
+                       hidden, epsilon, stream),
+                   "layer output");
+    runner.launches += 1;
+    std::swap(current, other);
+  }
+  int *host_results = runner.host_results.get<int>();
+  if (last_count > 0) {
+    require_launch(launch_prefill_last_rows(runner.q_final.get(), device + layout.last_rows,
+                                            device + layout.last_slots, last_count, hidden,
+                                            runner.q_last_rows.get(), runner.hidden_by_slot.get(),
+                                            stream),
+                   "prefill hand-off rows");
+    const LinearPlan head =
+        plan_bf16_linear(runner.q_last_rows.get(), runner.weights.token_embedding, last_count,
+                         hidden, config.vocabulary_size, 1);
+    require_launch(launch_linear_argmax(head, nullptr, nullptr, best, runner.device_error, stream),
+                   "BF16 LM head");
+    int *device_predictions = runner.step_results.get<int>() + 2 * runner.batch;
+    require_launch(launch_unpack_best(best, device_predictions, last_count, stream),
+                   "prefill argmax");
+    runner.launches += 3;
+    require_cuda(cudaMemcpyAsync(host_results, device_predictions, sizeof(int) * last_count,
+                                 cudaMemcpyDeviceToHost, stream),
+                 "copy prefill predictions");
+  }
+  require_cuda(cudaMemcpyAsync(host_results + maximum_rows, runner.device_error, sizeof(int),
+                               cudaMemcpyDeviceToHost, stream),
+               "copy device error word");
+  require_cuda(cudaEventRecord(runner.stop_event, stream), "record prefill end");
+  require_cuda(cudaStreamSynchronize(stream), "synchronize prefill step");
+  require_cuda(cudaEventElapsedTime(&runner.last_verify_ms, runner.start_event, runner.stop_event),
+               "read prefill step time");
+  runner.last_verify_launches = runner.launches;
+  if (host_results[maximum_rows] != 0) {
+    const int code = host_results[maximum_rows];
+    cudaMemsetAsync(runner.device_error, 0, sizeof(int), stream);
+    throw Failure{"a kernel wait ran out during prefill (code " + std::to_string(code) + ")"};
+  }
+  int next = 0;
+  for (size_t index = 0; index < segments.size(); ++index) {
+    if (complete[index])
+      predictions[index] = host_results[next++];
+    runner.slot_positions[static_cast<size_t>(segments[index].slot)] += segments[index].count;
+  }
+}
+
 void draft_step(Runner &runner, const int *last_tokens, const int *slots, const int *forced,
                 int requests, int depth, int *proposals_out) {
   if (!runner.has_assistant || last_tokens == nullptr || slots == nullptr || requests <= 0 ||
@@ -1893,6 +2368,11 @@ extern "C" int carat_b200_runner_set_bf16_weights(carat_b200_runner *runner,
     }
     runner->bf16_layers.assign(layers, layers + layer_count);
     runner->prefill_plans.clear();
+    runner->packed_prefill = packed_prefill_takes(*runner);
+    if (runner->packed_prefill) {
+      prepare_packed_prefill(*runner);
+      return;
+    }
     if (runner->p_normed.get() == nullptr) {
       const size_t rows = maximum_rows;
       runner->p_normed.allocate(rows * runner->config.hidden_size * 2);
@@ -1942,6 +2422,40 @@ extern "C" int carat_b200_runner_prefill_slots_chunks(
       }
       has_prediction[request] = 0;
       predictions[request] = -1;
+    }
+    if (runner->packed_prefill) {
+      // Steps of up to packed_prefill_rows rows, the requests' remaining rows in order.
+      std::vector<int> at = begin;
+      int request = 0;
+      while (request < requests) {
+        std::vector<int> step_tokens;
+        std::vector<PrefillSegment> segments;
+        std::vector<bool> complete;
+        std::vector<int> owners;
+        while (request < requests &&
+               static_cast<int>(step_tokens.size()) < packed_prefill_rows) {
+          const size_t r = static_cast<size_t>(request);
+          const int count = std::min(end[r] - at[r], packed_prefill_rows -
+                                                         static_cast<int>(step_tokens.size()));
+          segments.push_back(packed_segment(*runner, slots[request], at[r], count));
+          step_tokens.insert(step_tokens.end(), token_ids[request] + at[r],
+                             token_ids[request] + at[r] + count);
+          at[r] += count;
+          complete.push_back(at[r] == token_counts[request]);
+          owners.push_back(request);
+          if (at[r] == end[r])
+            ++request;
+        }
+        std::vector<int> next(segments.size(), -1);
+        prefill_rows_step(*runner, step_tokens, segments, complete, next);
+        for (size_t index = 0; index < segments.size(); ++index) {
+          if (complete[index]) {
+            has_prediction[owners[index]] = 1;
+            predictions[owners[index]] = next[index];
+          }
+        }
+      }
+      return;
     }
     // Walk the chunks in steps. A step is a list of (request, eight-token piece) entries of one
     // common depth (rows of different entries never mix in bf16, so the grouping does not change

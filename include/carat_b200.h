@@ -702,9 +702,10 @@ CARAT_B200_API int carat_b200_runner_set_bf16_weights(carat_b200_runner *runner,
  * Replaces Gemma4BatchModelRunner::prefill_slots_chunks (and, with one slot, prefill_slot_chunk;
  * with chunk_tokens >= every remainder, prefill_slots_suffix's result for a cold cache):
  * include/carat/batch_model_runner.h:37-47, cuda/batch_model_runner.cu:1066-1125,1230-1355.
- * Inside, a chunk is walked in steps of at most eight tokens per request through the same
- * attention kernels the verify step uses; rows of different requests never mix in bf16, so the
- * walk does not change results. Needs carat_b200_runner_set_bf16_weights. */
+ * Inside, the chunks' rows are packed into forwards of up to 2,048 rows (models whose attention
+ * shapes the packed path does not take, head_dim 64 for one, walk them eight tokens a request at a
+ * time); rows of different requests never mix in bf16, so the cut does not change results. Needs
+ * carat_b200_runner_set_bf16_weights. */
 CARAT_B200_API int carat_b200_runner_prefill_slots_chunks(
     carat_b200_runner *runner, const int *slots, const int *const *token_ids,
     const int *token_counts, int requests, int chunk_tokens, int *predictions,

@@ -1,0 +1,74 @@
+"""Packed BF16 prefill steps (any number of rows of several prompts in one forward) at the sizes
+where they can go wrong: query tiles and 128-position key tiles that are partly filled, prompts
+around the window and around the 256 rows from which the linears run on CTA pairs, slots whose rings
+hold an earlier, longer prompt. A row's result depends on its position and the keys it sees only, so
+every cut of a prompt has to leave the same bytes; against the CPU oracle the bar is the one of
+test_prefill_bf16_gpu.py.
+"""
+import pytest
+import torch
+
+import helpers
+from helpers import rms_relative_error
+from oracle import carat_semantics as cs
+from test_prefill_bf16_gpu import build, prompts
+
+pytestmark = pytest.mark.gpu
+
+# Two and four query heads a KV head of 256, eight of 512.
+CONFIG = cs.ModelConfig(256, 512, 2048, 256, 1024, 1e-6,
+                        [cs.LayerConfig("sliding", 4, 2, 256, 1e4, False),
+                         cs.LayerConfig("sliding", 4, 1, 256, 1e4, False),
+                         cs.LayerConfig("global", 8, 1, 512, 1e6, True)])
+
+
+def state(config, device, slot, length):
+    rows = []
+    for index in range(len(config.layers)):
+        capacity = config.capacity(index)
+        for cache in (device.key_cache(index, capacity), device.value_cache(index, capacity)):
+            rows.append(cache[slot][:, :min(length, capacity)].contiguous().view(torch.int16))
+    rows.append(device.target_hidden_slots()[slot].view(torch.int16))
+    return rows
+
+
+@pytest.mark.parametrize("length", [1, 16, 63, 129, 256, 257, 321, 640, 1000])
+def test_every_cut_of_a_prompt_leaves_the_same_bytes(cuda_device, length):
+    text = prompts(CONFIG, [length], seed=length)[0]
+    other = prompts(CONFIG, [1000, 300], seed=5)
+    _, device = build(CONFIG, 4)
+    first = device.prefill_slot(0, text, chunk_tokens=1024)
+    wanted = state(CONFIG, device, 0, length)
+    # In pieces of 37 behind a longer prompt that used the slot before.
+    device.prefill_slot(1, other[0], chunk_tokens=1024)
+    assert device.prefill_slot(1, text, chunk_tokens=37) == first
+    # Between two other prompts in one step, then in pieces of 130 beside one.
+    device.prefill_slots_chunks([2, 3], [other[1], text], 1000)
+    cuts = [1, 3]
+    if length > 130:
+        device.reset_slot(2)
+        device.reset_slot(0)
+        got = None
+        while got is None:
+            got = device.prefill_slots_chunks([0, 2], [text, other[0]], 130)[0]
+        assert got == first
+        cuts.append(0)
+    for slot in cuts:
+        for have, want in zip(state(CONFIG, device, slot, length), wanted):
+            assert torch.equal(have, want), (length, slot)
+
+
+def test_long_steps_match_the_oracle(cuda_device):
+    lengths = [300, 517, 90]
+    texts = prompts(CONFIG, lengths, seed=11)
+    oracle, device = build(CONFIG, 3)
+    wanted = [oracle.prefill_slot_fp8(slot, text, chunk=8) for slot, text in enumerate(texts)]
+    got = device.prefill_slots_chunks([0, 1, 2], texts, 1024)    # 907 rows in one step
+    assert sum(a != b for a, b in zip(got, wanted)) <= 1          # near-ties only
+    for index in range(len(CONFIG.layers)):
+        capacity = CONFIG.capacity(index)
+        keys, values = device.key_cache(index, capacity), device.value_cache(index, capacity)
+        for slot in range(3):
+            assert rms_relative_error(keys[slot], oracle.keys[index][slot]) < 2e-2
+            assert rms_relative_error(values[slot], oracle.values[index][slot]) < 2e-2
+            assert helpers.cosine(keys[slot], oracle.keys[index][slot]) > 0.999
