@@ -37,7 +37,7 @@ inline bool pdl_enabled() {
   return enabled;
 }
 
-// The same for a grid of clusters of `cluster` CTAs.
+// A grid of clusters of `cluster` CTAs, outside the chain: an ordinary launch.
 template <typename... KernelArgs, typename... Args>
 cudaError_t launch_clustered(void (*kernel)(KernelArgs...), dim3 grid, dim3 block,
                              size_t shared_bytes, cudaStream_t stream, unsigned int cluster,
@@ -47,20 +47,13 @@ cudaError_t launch_clustered(void (*kernel)(KernelArgs...), dim3 grid, dim3 bloc
   config.blockDim = block;
   config.dynamicSmemBytes = shared_bytes;
   config.stream = stream;
-  cudaLaunchAttribute attributes[2];
-  unsigned int count = 0;
-  attributes[count].id = cudaLaunchAttributeClusterDimension;
-  attributes[count].val.clusterDim.x = cluster;
-  attributes[count].val.clusterDim.y = 1;
-  attributes[count].val.clusterDim.z = 1;
-  ++count;
-  if (pdl_enabled()) {
-    attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attributes[count].val.programmaticStreamSerializationAllowed = 1;
-    ++count;
-  }
-  config.attrs = attributes;
-  config.numAttrs = count;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = cluster;
+  attribute.val.clusterDim.y = 1;
+  attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
   return cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
 }
 

@@ -12,6 +12,12 @@
 // Above 256 rows (BF16 prefill) the same kernel is an ordinary tiled GEMM: the row tiles of a
 // feature tile are dealt to neighbouring pairs, so its weights come from HBM once and then from L2.
 //
+// The kernel stands outside the chain of programmatic dependent launches: it neither starts before
+// the previous grid has ended nor lets the next one start before it has. Overlapped with large
+// grids of small CTAs on both sides, launches of clusters stopped making progress now and then
+// (every few thousand launches; CTAs of a neighbour that wait for this grid can fill the SMs its
+// clusters still need). The overlap is worth one to two microseconds of a launch of 40 to 600.
+//
 // Roles per CTA: warp 0 requests tiles by TMA (no multicast; both CTAs' copies complete on the
 // leader's barrier), warp 1 of the leader issues the MMAs, warps 2-5 of both finish their 128
 // features x rows from their own tensor memory. Two accumulators, so a tile's epilogue overlaps
@@ -156,7 +162,6 @@ pair_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
   const int first_item = static_cast<int>(blockIdx.x) / 2;
   const int item_stride = static_cast<int>(gridDim.x) / 2;
 
-  grid_dependency_launch();
   if (threadIdx.x == 0) {
     for (uint32_t stage = 0; stage < stages; ++stage) {
       ptx::mbarrier_init(full_bar + 8U * stage, 1);
@@ -202,22 +207,6 @@ pair_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
       uint32_t stage = 0;
       uint32_t phase = 0;
       bool healthy = true;
-      // The weights are static: the first ring of weight tiles is requested before the grid this
-      // launch depends on has finished; the activation tiles of those stages follow once it has.
-      int early = 0;
-      if (first_item < items) {
-        const WorkItem item = decode_item(args, first_item / shape.row_tiles);
-        early = min(item.k_count, shape.stages);
-        for (int block = 0; block < early; ++block) {
-          if (rank == 0)
-            ptx::mbarrier_arrive_expect_tx(full_bar + 8U * block, pair_bytes);
-          pair_load_2d(weight_tiles + block * weight_bytes, &weight_map,
-                       (item.k_begin + block) * block_bytes,
-                       item.tile * pair_features + weight_row, leader_full + 8U * block,
-                       weight_policy);
-        }
-      }
-      grid_dependency_wait();
       for (int index = first_item; index < items && healthy; index += item_stride) {
         const int unit = shape.row_tiles == 1 ? index : index / shape.row_tiles;
         const WorkItem item = decode_item(args, unit);
@@ -225,20 +214,16 @@ pair_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
         const int y_input = (index - unit * shape.row_tiles) * shape.tile_rows + input_row;
         int k_byte = item.k_begin * block_bytes;
         for (int block = 0; block < item.k_count; ++block, k_byte += block_bytes) {
-          const uint32_t full = leader_full + 8U * stage;
-          if (early > 0) {
-            --early;     // this stage's weight tile is already on its way
-          } else {
-            if (!ptx::mbarrier_wait_fast(empty_bar + 8U * stage, phase ^ 1U)) {
-              healthy = false;
-              atomicExch(args.device_error, 1);
-              break;
-            }
-            if (rank == 0)
-              ptx::mbarrier_arrive_expect_tx(full_bar + 8U * stage, pair_bytes);
-            pair_load_2d(weight_tiles + stage * weight_bytes, &weight_map, k_byte, y_weight, full,
-                         weight_policy);
+          if (!ptx::mbarrier_wait_fast(empty_bar + 8U * stage, phase ^ 1U)) {
+            healthy = false;
+            atomicExch(args.device_error, 1);
+            break;
           }
+          const uint32_t full = leader_full + 8U * stage;
+          if (rank == 0)
+            ptx::mbarrier_arrive_expect_tx(full_bar + 8U * stage, pair_bytes);
+          pair_load_2d(weight_tiles + stage * weight_bytes, &weight_map, k_byte, y_weight, full,
+                       weight_policy);
           pair_load_2d(input_tiles + stage * input_bytes, &input_map, k_byte, y_input, full,
                        reuse_policy);
           if (++stage == stages) {
@@ -322,7 +307,6 @@ pair_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
     const int quarter = warp & 3;  // TMEM lane group this warp may read
     [[maybe_unused]] const int epilogue_thread = (warp - 2) * 32 + lane;
     const uint32_t leader_acc_empty = in_leader(acc_empty_bar);
-    grid_dependency_wait();
     float scale = 1.0F;
     if constexpr (mode != 1 && !wide)
       scale = args.input_scale[0] * args.weight_scale[0];
