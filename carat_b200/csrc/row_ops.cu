@@ -154,7 +154,9 @@ __device__ __forceinline__ Pack8 round_bf16x8(const Pack8 &values, uint4 *packed
 // exactly like a separate finishing kernel. The loads of all groups are issued together, a few
 // pieces at a time (as many as the registers hold): a loop that loads and adds group by group, or
 // piece by piece, pays one L2 round trip per turn.
-template <int chunks>
+// `many`: the grid has several CTAs a SM, which hide each other's round trips; a single piece at a
+// time then keeps the registers down to what two CTAs a SM may have.
+template <int chunks, bool many = false>
 __device__ __forceinline__ void load_source(const RowArguments &a, size_t row, int column_base,
                                             int column_end, size_t rows, float partial_scale,
                                             Pack8 (&values)[chunks]) {
@@ -167,7 +169,7 @@ __device__ __forceinline__ void load_source(const RowArguments &a, size_t row, i
     }
     return;
   }
-  constexpr int batch = chunks <= 1 ? 8 : chunks <= 2 ? 4 : chunks <= 4 ? 2 : 1;
+  constexpr int batch = many ? 1 : chunks <= 1 ? 8 : chunks <= 2 ? 4 : chunks <= 4 ? 2 : 1;
   int pieces = a.splits;
   if (a.valid_splits != nullptr)
     pieces = min(pieces, a.valid_splits[row / a.rows_per_group]);
@@ -222,8 +224,12 @@ __device__ __forceinline__ void load_source(const RowArguments &a, size_t row, i
 // store (needs every CTA resident at once). true: the kernel stops after the maximum, leaving the
 // bf16 rows in a.pass_rows, and quantize_rows_kernel finishes; used when there are more rows than
 // the device holds CTAs (the scratch words must then have been cleared by the caller).
-template <RowMode mode, int chunks, bool two_launches>
-__global__ void __launch_bounds__(row_threads, (mode == RowMode::geglu && chunks <= 4) ? 2 : 1)
+//
+// `many` = true (bf16 rows only, more rows than SMs: BF16 prefill): two CTAs a SM instead of one
+// with every load in flight. The norm weights then come when they are needed, from L1 or L2.
+template <RowMode mode, int chunks, bool two_launches, bool many = false>
+__global__ void
+__launch_bounds__(row_threads, (many || (mode == RowMode::geglu && chunks <= 4)) ? 2 : 1)
 row_kernel(RowArguments a) {
   __shared__ float scratch[2 * row_warps];
   int parity = 0;
@@ -249,7 +255,7 @@ row_kernel(RowArguments a) {
     const int column = column_base + (chunk * row_threads + static_cast<int>(threadIdx.x)) * 8;
     weight_raw[chunk] = make_uint4(0, 0, 0, 0);
     next_weight_raw[chunk] = make_uint4(0, 0, 0, 0);
-    if (column < column_end) {
+    if (column < column_end && !many) {
       if constexpr (one_norm || two_norms)
         weight_raw[chunk] = *reinterpret_cast<const uint4 *>(a.norm_weight + column);
       if constexpr (two_norms)
@@ -300,7 +306,7 @@ row_kernel(RowArguments a) {
           residual_raw[chunk] = *reinterpret_cast<const uint4 *>(a.residual + row * width + column);
       }
     }
-    load_source<chunks>(a, row, column_base, column_end, rows, partial_scale, values);
+    load_source<chunks, many>(a, row, column_base, column_end, rows, partial_scale, values);
   } else if constexpr (mode == RowMode::embed_norm || mode == RowMode::embed_concat) {
     // embed_concat: `width` is the concatenated width, scaled embedding row then the carried
     // hidden state.
@@ -441,6 +447,8 @@ row_kernel(RowArguments a) {
       const int column = column_base + (chunk * row_threads + static_cast<int>(threadIdx.x)) * 8;
       if (column >= column_end)
         continue;
+      if constexpr (many)
+        weight_raw[chunk] = *reinterpret_cast<const uint4 *>(a.norm_weight + column);
       const Pack8 weights = unpack_bf16x8(weight_raw[chunk]);
       Pack8 result;
       if constexpr (two_norms) {
@@ -485,6 +493,8 @@ row_kernel(RowArguments a) {
       const int column = column_base + (chunk * row_threads + static_cast<int>(threadIdx.x)) * 8;
       if (column >= column_end)
         continue;
+      if constexpr (many)
+        next_weight_raw[chunk] = *reinterpret_cast<const uint4 *>(a.next_norm_weight + column);
       const Pack8 weights = unpack_bf16x8(next_weight_raw[chunk]);
       Pack8 result;
 #pragma unroll
@@ -623,7 +633,16 @@ int launch_rows_chunks(const RowArguments &arguments, int ctas, cudaStream_t str
   if (resident_limit <= 0)
     return -10;
   if (arguments.fp8_output == nullptr) {
-    // No quantisation, so no grid barrier: any number of CTAs, plain launch.
+    // No quantisation, so no grid barrier: any number of CTAs, plain launch. 2,048 rows of 5,376
+    // (three fp32 pieces in, two bf16 rows out): 53 us with one CTA a SM, 45 with two.
+    if constexpr (chunks <= 2 && (mode == RowMode::post_attention || mode == RowMode::layer_output)) {
+      if (ctas > 2 * device_multiprocessors()) {
+        const cudaError_t many_status =
+            launch_chained(row_kernel<mode, chunks, false, true>, dim3(static_cast<unsigned>(ctas)),
+                           dim3(row_threads), 0, stream, false, arguments);
+        return many_status == cudaSuccess ? 0 : -11;
+      }
+    }
     const cudaError_t status =
         launch_chained(row_kernel<mode, chunks, false>, dim3(static_cast<unsigned>(ctas)),
                        dim3(row_threads), 0, stream, false, arguments);
@@ -670,8 +689,14 @@ template <RowMode mode> int launch_rows(RowArguments arguments, int rows, cudaSt
   if constexpr (mode == RowMode::geglu) {
     // Wide rows: two CTAs a row when the halves stay multiples of eight columns and the grid
     // still fits the device at once (checked by launch_rows_chunks).
-    if (arguments.width >= 8192 && arguments.width % 16 == 0 && rows <= 148)
+    if (bf16_only && rows > 148) {
+      // No grid to keep resident: parts of at most two column groups a thread, two CTAs a SM.
+      // 2,048 rows of 21,504: 107 us in one part, 86 in three.
+      while (arguments.width / parts > 2 * row_threads * 8 || arguments.width % (8 * parts) != 0)
+        ++parts;
+    } else if (arguments.width >= 8192 && arguments.width % 16 == 0 && rows <= 148) {
       parts = 2;   // 2 * 148 CTAs of the two-per-SM variant fit
+    }
   }
   for (; parts >= 1; --parts) {
     arguments.parts = parts;
