@@ -7,15 +7,15 @@
 // Same swapped-operand weight stream as the e4m3 linear (128 output features = UMMA M, padded
 // activation rows = UMMA N, persistent CTAs walking tile x K-piece items), with one more stage
 // between TMA and the tensor core: the 4-bit codes cannot feed tcgen05.mma together with bf16
-// activations, so eight warps turn every [128 features x 128 K] tile of codes (8 KB, plus its 128
+// activations, so two or three groups of four warps turn every [128 features x 128 K] tile of codes (8 KB, plus its 128
 // group scales) into bf16 and store it into tensor memory (tcgen05.st), where the MMA warp takes
 // it as the A operand (kind::f16, A in TMEM) against the bf16 activation boxes in shared memory.
 // Keeping the converted weights out of shared memory matters: written there and read back by the
 // tensor core they cost 64 KB of shared-memory traffic per K block on top of the 72 KB of TMA
 // writes and B-operand reads, and the kernel was bound by shared-memory bandwidth (measured: no
 // change when either TMA stream was switched off). Rings: codes + scales (TMA, deep, small),
-// activations (TMA from L2), converted weights (four TMEM buffers of 64 columns, filled by two
-// groups of four warps on alternate K blocks). The codes are read from HBM exactly once; that is
+// activations (TMA from L2), converted weights (four TMEM buffers of 64 columns, filled by two or
+// three groups of four warps on consecutive K blocks). The codes are read from HBM exactly once; that is
 // half the bytes of the e4m3 weights, but the kernel is bound on the SM: at 128 padded rows the
 // eight bf16 MMAs of a K block keep the tensor pipe busy about 700 cycles (an e4m3 MMA consumes 32
 // bytes of a weight row, a bf16 MMA over 4-bit codes 8), and below 64 rows the conversion (shift,
@@ -32,15 +32,18 @@
 namespace carat_b200 {
 namespace {
 
-constexpr int int4_threads = 480;        // warp 0 codes TMA, 1 MMA, 2 activations TMA, 3-6 epilogue,
-constexpr int first_convert_warp = 7;    // 7-14 convert
-constexpr int convert_warps = 8;
+constexpr int first_convert_warp = 7;    // warp 0 codes TMA, 1 MMA, 2 activations TMA, 3-6 epilogue
 constexpr int code_tile_bytes = tile_features * 64;          // 128 features x 128 codes
 constexpr int scale_tile_bytes = tile_features * 2;
 constexpr int weight_buffers = 4;
 constexpr int weight_columns = tile_k_elements / 2;          // TMEM columns of one converted K block
 
 template <int padded_rows> struct Layout {
+  // Groups of four converting warps, on consecutive K blocks. Where the conversion is the limit a
+  // third group fills the pipes better (5376 -> 43008, 24 rows 47.0 -> 42.1 us, 64 rows 49.6 ->
+  // 46.8); beside MMAs of 128 rows it only takes issue slots from them (57.0 -> 57.5).
+  static constexpr int convert_groups = padded_rows >= 128 ? 2 : 3;
+  static constexpr int threads = (first_convert_warp + 4 * convert_groups) * 32;
   static constexpr int input_box_bytes = padded_rows * 128;  // rows x 64 bf16
   static constexpr int input_stage_bytes = 2 * input_box_bytes;
   static constexpr int input_stages = padded_rows >= 128 ? 4 : 6;
@@ -81,7 +84,7 @@ __device__ __forceinline__ void convert_word(uint32_t word, __nv_bfloat162 scale
 }
 
 template <int padded_rows, int mode>
-__global__ void __launch_bounds__(int4_threads, 1)
+__global__ void __launch_bounds__(Layout<padded_rows>::threads, 1)
 int4_linear_kernel(const __grid_constant__ CUtensorMap code_map,
                    const __grid_constant__ CUtensorMap scale_map,
                    const __grid_constant__ CUtensorMap input_map, const KernelArguments args,
@@ -124,14 +127,14 @@ int4_linear_kernel(const __grid_constant__ CUtensorMap code_map,
     abort_word = 0;
     for (int stage = 0; stage < L::code_stages; ++stage) {
       ptx::mbarrier_init(code_full + 8U * stage, 1);
-      ptx::mbarrier_init(code_empty + 8U * stage, convert_warps / 2);
+      ptx::mbarrier_init(code_empty + 8U * stage, 4);
     }
     for (int stage = 0; stage < L::input_stages; ++stage) {
       ptx::mbarrier_init(input_full + 8U * stage, 1);
       ptx::mbarrier_init(input_empty + 8U * stage, 1);
     }
     for (int buffer = 0; buffer < weight_buffers; ++buffer) {
-      ptx::mbarrier_init(weight_full + 8U * buffer, convert_warps / 2);
+      ptx::mbarrier_init(weight_full + 8U * buffer, 4);
       ptx::mbarrier_init(weight_empty + 8U * buffer, 1);
     }
     for (int buffer = 0; buffer < 2; ++buffer) {
@@ -278,9 +281,9 @@ int4_linear_kernel(const __grid_constant__ CUtensorMap code_map,
     }
   } else if (warp >= first_convert_warp) {
     // Thread -> feature row: a warp may touch only its own quarter of the TMEM lanes (warp index
-    // mod 4), lane = feature row. The eight warps form two groups of four that take alternate K
-    // blocks, so that on every scheduler one warp is converting while the other waits, loads or
-    // stores (in lockstep all eight hit the integer and bf16 pipes at the same moment and leave
+    // mod 4), lane = feature row. The warps form groups of four that take consecutive K blocks, so
+    // that on every scheduler one warp is converting while the other waits, loads or
+    // stores (in lockstep all of them hit the integer and bf16 pipes at the same moment and leave
     // them idle the rest of the time). Code tiles arrive with the 64-byte swizzle (16-byte chunk
     // index xor bits 1-2 of the row), so the reads of a quarter warp touch eight bank groups.
     const int row = (warp & 3) * 32 + lane;
@@ -295,11 +298,11 @@ int4_linear_kernel(const __grid_constant__ CUtensorMap code_map,
       total_blocks += decode_item(args, index).k_count;
     Cursor<L::code_stages> code_cursor;
     Cursor<weight_buffers> weight_cursor;
-    if (group == 1) {
+    for (int ahead = 0; ahead < group; ++ahead) {
       code_cursor.advance();
       weight_cursor.advance();
     }
-    for (int block = group; block < total_blocks; block += 2) {
+    for (int block = group; block < total_blocks; block += L::convert_groups) {
       const bool ready =
           ptx::mbarrier_wait_checked(code_full + 8U * code_cursor.stage, code_cursor.phase, abort_flag,
                        args.device_error, 65) &&
@@ -337,10 +340,11 @@ int4_linear_kernel(const __grid_constant__ CUtensorMap code_map,
         ptx::mbarrier_arrive(weight_full + 8U * weight_cursor.stage);
         ptx::mbarrier_arrive(code_empty + 8U * code_cursor.stage);
       }
-      code_cursor.advance();
-      code_cursor.advance();
-      weight_cursor.advance();
-      weight_cursor.advance();
+#pragma unroll
+      for (int ahead = 0; ahead < L::convert_groups; ++ahead) {
+        code_cursor.advance();
+        weight_cursor.advance();
+      }
     }
   } else {
     const int quarter = warp & 3;  // TMEM lane group this warp may read
@@ -536,7 +540,7 @@ int launch_variant(const Int4LinearPlan &plan, const KernelArguments &arguments,
                     arguments.tail_tiles * arguments.tail_splits;
   const int ctas = items < schedule.ctas ? items : schedule.ctas;
   return launch_chained(int4_linear_kernel<padded_rows, mode>, dim3(static_cast<unsigned>(ctas)),
-                        dim3(int4_threads), dynamic_bytes, stream, false, schedule.weight_map,
+                        dim3(Layout<padded_rows>::threads), dynamic_bytes, stream, false, schedule.weight_map,
                         plan.scale_map, schedule.input_map, arguments,
                         plan.group_shift) == cudaSuccess
              ? 0
