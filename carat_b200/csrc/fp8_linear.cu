@@ -604,40 +604,71 @@ fp8_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
   }
 }
 
-__global__ void finalize_split_k_kernel(const float *partial, const float *input_scale,
-                                        const float *weight_scale, __nv_bfloat16 *output,
-                                        int splits, size_t elements) {
+// output[row, first_column + c] = bf16(scale * sum over pieces of partial[piece, row, c]), pieces
+// added in order. Latency is all of it (a few MB that the linear has just left in L2), so a thread
+// takes eight columns in 16-byte accesses and has four pieces in flight: 5.4 us for 3 x 216 x 5376
+// sums where one column a thread and turn takes 8.9, 4.7 for 120 rows (6.5).
+__global__ void __launch_bounds__(256)
+finalize_vector_kernel(const float *partial, const float *input_scale, const float *weight_scale,
+                       __nv_bfloat16 *output, int pieces, int rows, int width, int output_width,
+                       int first_column) {
   grid_dependency_launch();
+  const int groups = width / 8;
+  const int index = static_cast<int>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (index >= rows * groups)
+    return;
+  const int row = index / groups;
+  const int column = (index - row * groups) * 8;
+  const size_t piece_elements = static_cast<size_t>(rows) * width;
+  const float *source = partial + static_cast<size_t>(row) * width + column;
   grid_dependency_wait();
   const float scale = input_scale != nullptr ? input_scale[0] * weight_scale[0] : 1.0F;
-  for (size_t index = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-       index < elements; index += static_cast<size_t>(blockDim.x) * gridDim.x) {
-    // Four pieces a round trip, added in piece order.
-    float sum = 0.0F;
-    for (int first = 0; first < splits; first += 4) {
-      float piece[4];
+  float sum[8] = {0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F};
+  for (int first = 0; first < pieces; first += 4) {
+    float4 low[4];
+    float4 high[4];
 #pragma unroll
-      for (int offset = 0; offset < 4; ++offset)
-        piece[offset] = first + offset < splits
-                            ? partial[static_cast<size_t>(first + offset) * elements + index]
-                            : 0.0F;
-#pragma unroll
-      for (int offset = 0; offset < 4; ++offset)
-        if (first + offset < splits)
-          sum += piece[offset];
+    for (int offset = 0; offset < 4; ++offset) {
+      if (first + offset < pieces) {
+        const auto *vectors =
+            reinterpret_cast<const float4 *>(source + (first + offset) * piece_elements);
+        low[offset] = __ldcg(vectors);
+        high[offset] = __ldcg(vectors + 1);
+      }
     }
-    output[index] = __float2bfloat16_rn(sum * scale);
+#pragma unroll
+    for (int offset = 0; offset < 4; ++offset) {
+      if (first + offset < pieces) {
+        sum[0] += low[offset].x;
+        sum[1] += low[offset].y;
+        sum[2] += low[offset].z;
+        sum[3] += low[offset].w;
+        sum[4] += high[offset].x;
+        sum[5] += high[offset].y;
+        sum[6] += high[offset].z;
+        sum[7] += high[offset].w;
+      }
+    }
   }
+  __nv_bfloat162 packed[4];
+#pragma unroll
+  for (int pair = 0; pair < 4; ++pair)
+    packed[pair] = __floats2bfloat162_rn(sum[2 * pair] * scale, sum[2 * pair + 1] * scale);
+  *reinterpret_cast<uint4 *>(output + static_cast<size_t>(row) * output_width + first_column +
+                             column) = *reinterpret_cast<const uint4 *>(packed);
 }
 
-// output[row, first_column + c] = bf16(scale * sum over pieces of partial[piece, row, c]).
-__global__ void finalize_tail_kernel(const float *partial, const float *input_scale,
-                                     const float *weight_scale, __nv_bfloat16 *output, int pieces,
-                                     int rows, int tail_width, int output_width, int first_column) {
+// The same, one column a turn: for calls so small that every thread has one column at most (5 rows
+// of 5376: 11.35 us with the linear, 11.55 with the other), and for widths or pointers that do not
+// allow 16-byte accesses.
+__global__ void finalize_column_kernel(const float *partial, const float *input_scale,
+                                       const float *weight_scale, __nv_bfloat16 *output,
+                                       int pieces, int rows, int width, int output_width,
+                                       int first_column) {
   grid_dependency_launch();
   grid_dependency_wait();
   const float scale = input_scale != nullptr ? input_scale[0] * weight_scale[0] : 1.0F;
-  const size_t elements = static_cast<size_t>(rows) * tail_width;
+  const size_t elements = static_cast<size_t>(rows) * width;
   for (size_t index = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
        index < elements; index += static_cast<size_t>(blockDim.x) * gridDim.x) {
     float sum = 0.0F;
@@ -653,8 +684,8 @@ __global__ void finalize_tail_kernel(const float *partial, const float *input_sc
         if (first + offset < pieces)
           sum += piece[offset];
     }
-    const size_t row = index / tail_width;
-    const size_t column = index - row * tail_width;
+    const size_t row = index / width;
+    const size_t column = index - row * width;
     output[row * output_width + first_column + column] = __float2bfloat16_rn(sum * scale);
   }
 }
@@ -931,15 +962,9 @@ int launch_linear_bf16(const LinearPlan &plan, const float *input_scale, const f
     if (status != 0)
       return status;
     const int tail_width = plan.tail_columns();
-    const size_t elements = static_cast<size_t>(plan.rows) * tail_width;
-    const int blocks = static_cast<int>((elements + 255) / 256);
-    return launch_chained(finalize_tail_kernel, dim3(blocks < 1184 ? blocks : 1184), dim3(256), 0,
-                          stream, false, static_cast<const float *>(partial), input_scale,
-                          weight_scale, static_cast<__nv_bfloat16 *>(bf16_output),
-                          plan.tail_splits, plan.rows, tail_width, plan.output_width,
-                          plan.output_width - tail_width) == cudaSuccess
-               ? 0
-               : -11;
+    return launch_linear_finalize(partial, input_scale, weight_scale, bf16_output,
+                                  plan.tail_splits, plan.rows, tail_width, plan.output_width,
+                                  plan.output_width - tail_width, stream);
   }
   if (plan.splits == 1) {
     KernelArguments arguments = base_arguments(plan, device_error, false);
@@ -951,12 +976,31 @@ int launch_linear_bf16(const LinearPlan &plan, const float *input_scale, const f
   const int status = launch_linear_partial(plan, partial, device_error, stream);
   if (status != 0)
     return status;
-  const size_t elements = static_cast<size_t>(plan.rows) * plan.output_width;
-  const int blocks = static_cast<int>((elements + 255) / 256);
-  return launch_chained(finalize_split_k_kernel, dim3(blocks < 1184 ? blocks : 1184), dim3(256), 0,
-                        stream, false, static_cast<const float *>(partial), input_scale,
-                        weight_scale, static_cast<__nv_bfloat16 *>(bf16_output), plan.splits,
-                        elements) == cudaSuccess
+  return launch_linear_finalize(partial, input_scale, weight_scale, bf16_output, plan.splits,
+                                plan.rows, plan.output_width, plan.output_width, 0, stream);
+}
+
+int launch_linear_finalize(const float *partial, const float *input_scale,
+                           const float *weight_scale, void *bf16_output, int pieces, int rows,
+                           int width, int output_width, int first_column, cudaStream_t stream) {
+  auto *output = static_cast<__nv_bfloat16 *>(bf16_output);
+  const size_t elements = static_cast<size_t>(rows) * width;
+  const bool vectors = elements > 65536 && width % 8 == 0 && output_width % 8 == 0 && first_column % 8 == 0 &&
+                       reinterpret_cast<uintptr_t>(partial) % 16 == 0 &&
+                       reinterpret_cast<uintptr_t>(output) % 16 == 0 && elements / 8 < 0x7FFFFF00U;
+  if (vectors) {
+    const unsigned blocks = static_cast<unsigned>((elements / 8 + 255) / 256);
+    return launch_chained(finalize_vector_kernel, dim3(blocks), dim3(256), 0, stream, false, partial,
+                          input_scale, weight_scale, output, pieces, rows, width,
+                          output_width, first_column) == cudaSuccess
+               ? 0
+               : -11;
+  }
+  const size_t wanted = (elements + 255) / 256;
+  const unsigned blocks = static_cast<unsigned>(wanted < 1184 ? wanted : 1184);
+  return launch_chained(finalize_column_kernel, dim3(blocks), dim3(256), 0, stream, false, partial,
+                        input_scale, weight_scale, output, pieces, rows, width, output_width,
+                        first_column) == cudaSuccess
              ? 0
              : -11;
 }

@@ -102,6 +102,12 @@ int launch_linear_bf16_tail(const LinearPlan &plan, const float *input_scale,
                             int *device_error, cudaStream_t stream);
 std::size_t linear_tail_bytes(const LinearPlan &plan);
 
+// output[row, first_column + c] = bf16(scale * sum of partial[piece, row, c] in piece order), rows
+// of `width` sums into rows of output_width. Null scales multiply by one.
+int launch_linear_finalize(const float *partial, const float *input_scale,
+                           const float *weight_scale, void *bf16_output, int pieces, int rows,
+                           int width, int output_width, int first_column, cudaStream_t stream);
+
 // Leaves the unscaled fp32 partial sums [splits, rows, output_width] for a consumer that sums them.
 int launch_linear_partial(const LinearPlan &plan, float *partial, int *device_error,
                           cudaStream_t stream);

@@ -416,25 +416,6 @@ int4_linear_kernel(const __grid_constant__ CUtensorMap code_map,
   }
 }
 
-// output = bf16(sum of fp32 pieces); `first_column` / `piece_width` select a column range of the
-// output rows (the whole row for split-K, the tail columns for the K-cut tail round).
-__global__ void int4_finalize_kernel(const float *partial, __nv_bfloat16 *output, int pieces,
-                                     int rows, int piece_width, int output_width,
-                                     int first_column) {
-  grid_dependency_launch();
-  grid_dependency_wait();
-  const size_t elements = static_cast<size_t>(rows) * piece_width;
-  for (size_t index = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-       index < elements; index += static_cast<size_t>(blockDim.x) * gridDim.x) {
-    float sum = 0.0F;
-    for (int piece = 0; piece < pieces; ++piece)
-      sum += partial[static_cast<size_t>(piece) * elements + index];
-    const size_t row = index / piece_width;
-    const size_t column = index - row * piece_width;
-    output[row * output_width + first_column + column] = __float2bfloat16_rn(sum);
-  }
-}
-
 __device__ __forceinline__ float block_max_256(float value, float *scratch) {
   for (int offset = 16; offset > 0; offset >>= 1)
     value = fmaxf(value, __shfl_xor_sync(0xFFFFFFFFU, value, offset));
@@ -576,17 +557,6 @@ KernelArguments base_arguments(const LinearPlan &plan, int *device_error, bool s
   return arguments;
 }
 
-int launch_finalize(const float *partial, void *bf16_output, int pieces, int rows, int piece_width,
-                    int output_width, int first_column, cudaStream_t stream) {
-  const size_t elements = static_cast<size_t>(rows) * piece_width;
-  const int blocks = static_cast<int>((elements + 255) / 256);
-  return launch_chained(int4_finalize_kernel, dim3(blocks < 1184 ? blocks : 1184), dim3(256), 0,
-                        stream, false, partial, static_cast<__nv_bfloat16 *>(bf16_output), pieces,
-                        rows, piece_width, output_width, first_column) == cudaSuccess
-             ? 0
-             : -11;
-}
-
 std::size_t partial_bytes(const LinearPlan &plan) {
   if (plan.splits > 1)
     return sizeof(float) * static_cast<std::size_t>(plan.splits) * plan.rows * plan.output_width;
@@ -711,7 +681,7 @@ int launch_int4_linear_bf16(const Int4LinearPlan &plan, void *bf16_output, float
     if (status != 0)
       return status;
     const int tail_width = schedule.tail_tiles * tile_features;
-    return launch_finalize(partial, bf16_output, schedule.tail_splits, schedule.rows, tail_width,
+    return launch_linear_finalize(partial, nullptr, nullptr, bf16_output, schedule.tail_splits, schedule.rows, tail_width,
                            schedule.output_width, schedule.output_width - tail_width, stream);
   }
   if (schedule.splits == 1) {
@@ -722,7 +692,7 @@ int launch_int4_linear_bf16(const Int4LinearPlan &plan, void *bf16_output, float
   const int status = launch_int4_linear_partial(plan, partial, device_error, stream);
   if (status != 0)
     return status;
-  return launch_finalize(partial, bf16_output, schedule.splits, schedule.rows,
+  return launch_linear_finalize(partial, nullptr, nullptr, bf16_output, schedule.splits, schedule.rows,
                          schedule.output_width, schedule.output_width, 0, stream);
 }
 
