@@ -30,11 +30,12 @@ constexpr int tile_k_bytes = 128;   // one 128B swizzle atom of e4m3 per row
 constexpr int umma_k = 32;
 constexpr int linear_threads = 192; // warp 0 TMA, warp 1 MMA + TMEM, warps 2-5 epilogue
 constexpr int weight_tile_bytes = tile_features * tile_k_bytes;
-constexpr int shared_budget = 200 * 1024;
+constexpr int shared_budget = 220 * 1024;         // small CTAs of the next grid need a few KB beside it
+constexpr int gated_shared_budget = 200 * 1024;   // beside the gated epilogue's exchange buffers
 
-__host__ __device__ constexpr int stages_for(int padded_rows) {
+__host__ __device__ constexpr int stages_for(int padded_rows, int mode) {
   const int per_stage = weight_tile_bytes + padded_rows * tile_k_bytes;
-  const int fit = shared_budget / per_stage;
+  const int fit = (mode == 3 ? gated_shared_budget : shared_budget) / per_stage;
   return fit > 8 ? 8 : fit;
 }
 
@@ -104,13 +105,15 @@ template <int padded_rows, int mode, bool wide>
 __global__ void __launch_bounds__(linear_threads, 1)
 fp8_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
                   const __grid_constant__ CUtensorMap input_map, const KernelArguments args) {
-  constexpr int stages = stages_for(padded_rows);
+  constexpr int stages = stages_for(padded_rows, mode);
   constexpr int input_tile_bytes = padded_rows * tile_k_bytes;
   constexpr uint32_t stage_bytes = weight_tile_bytes + input_tile_bytes;
   constexpr uint32_t idesc = wide ? ptx::umma_idesc(1, 1, tile_features, padded_rows)
                                   : ptx::umma_idesc(0, 0, tile_features, padded_rows);
-  // Two accumulators; tensor-memory allocations are powers of two (192 padded rows take 512).
-  constexpr uint32_t tmem_columns = 2 * padded_rows < 32 ? 32 : 2 * padded_rows > 256 ? 512 : 2 * padded_rows;
+  // Two accumulators in an allocation of a power of two of columns.
+  constexpr uint32_t tmem_columns =
+      padded_rows <= 32 ? 64 : padded_rows <= 64 ? 128 : padded_rows <= 128 ? 256 : 512;
+  static_assert(tmem_columns >= 2 * padded_rows, "two accumulators");
 
   extern __shared__ unsigned char shared_raw[];
   __shared__ __align__(8) unsigned long long barriers[2 * stages + 4];
@@ -658,9 +661,10 @@ finalize_vector_kernel(const float *partial, const float *input_scale, const flo
                              column) = *reinterpret_cast<const uint4 *>(packed);
 }
 
-// The same, one column a turn: for calls so small that every thread has one column at most (5 rows
-// of 5376: 11.35 us with the linear, 11.55 with the other), and for widths or pointers that do not
-// allow 16-byte accesses.
+// The same, one column a turn: for widths or pointers that do not allow 16-byte accesses, and for
+// calls too small to give the other kernel a few blocks a SM (with the linear: 24 rows of 5376 in
+// three pieces 11.3 us against 12.1, 72 rows 12.9 against 13.4, 120 rows of 1024 in eighteen 10.3
+// against 12.0).
 __global__ void finalize_column_kernel(const float *partial, const float *input_scale,
                                        const float *weight_scale, __nv_bfloat16 *output,
                                        int pieces, int rows, int width, int output_width,
@@ -684,9 +688,12 @@ __global__ void finalize_column_kernel(const float *partial, const float *input_
         if (first + offset < pieces)
           sum += piece[offset];
     }
-    const size_t row = index / width;
-    const size_t column = index - row * width;
-    output[row * output_width + first_column + column] = __float2bfloat16_rn(sum * scale);
+    size_t destination = index;
+    if (width != output_width) {   // a division is a good part of a small call
+      const size_t row = index / width;
+      destination = row * output_width + first_column + (index - row * width);
+    }
+    output[destination] = __float2bfloat16_rn(sum * scale);
   }
 }
 
@@ -732,7 +739,7 @@ bool encode_byte_matrix(CUtensorMap *map, const void *base, uint64_t inner, uint
 
 template <int padded_rows, int mode, bool wide>
 int launch_variant(const LinearPlan &plan, const KernelArguments &arguments, cudaStream_t stream) {
-  constexpr int stages = stages_for(padded_rows);
+  constexpr int stages = stages_for(padded_rows, mode);
   constexpr int dynamic_bytes = stages * (weight_tile_bytes + padded_rows * tile_k_bytes) + 1024;
   static PerDeviceOnce configured;
   if (configured.run([] {
@@ -752,6 +759,10 @@ int launch_variant(const LinearPlan &plan, const KernelArguments &arguments, cud
              : -11;
 }
 
+// Rows in steps of 32: what a call loads, multiplies and holds in its ring is close to its rows.
+// With steps of 64 beyond 64, 216 rows (24 slots, nine proposals) filled 256 and left room for four
+// stages instead of five: e4m3 21504 -> 5376 35.5 us instead of 29.6, 5376 -> 43008 64.3 instead of
+// 49.6; 150 rows 50.8 instead of 46.9, 72 rows 41.8 instead of 40.3.
 template <int mode, bool wide>
 int launch_rows_bucket(const LinearPlan &plan, const KernelArguments &arguments,
                        cudaStream_t stream) {
@@ -760,10 +771,22 @@ int launch_rows_bucket(const LinearPlan &plan, const KernelArguments &arguments,
     return launch_variant<32, mode, wide>(plan, arguments, stream);
   case 64:
     return launch_variant<64, mode, wide>(plan, arguments, stream);
+  case 96:
+    if constexpr (mode != 3)
+      return launch_variant<96, mode, wide>(plan, arguments, stream);
+    return -12;
   case 128:
     return launch_variant<128, mode, wide>(plan, arguments, stream);
+  case 160:
+    if constexpr (mode != 3)
+      return launch_variant<160, mode, wide>(plan, arguments, stream);
+    return -12;
   case 192:
     return launch_variant<192, mode, wide>(plan, arguments, stream);
+  case 224:
+    if constexpr (mode != 3)
+      return launch_variant<224, mode, wide>(plan, arguments, stream);
+    return -12;
   case 256:
     return launch_variant<256, mode, wide>(plan, arguments, stream);
   default:
@@ -793,6 +816,7 @@ int launch_planned(const LinearPlan &plan, const KernelArguments &arguments, cud
 bool schedule_plain(LinearPlan *plan, int rows, int input_width, int output_width,
                     int requested_splits, int element_bytes) {
   schedule_linear(plan, rows, input_width, output_width, requested_splits, element_bytes);
+  plan->padded_rows = (rows + 31) / 32 * 32;
   if (rows > 256)
     return schedule_pairs(plan);
   if (plan->splits == 1 && plan->tiles >= plan->ctas / 2 && plan->k_blocks >= 32 &&
@@ -985,7 +1009,7 @@ int launch_linear_finalize(const float *partial, const float *input_scale,
                            int width, int output_width, int first_column, cudaStream_t stream) {
   auto *output = static_cast<__nv_bfloat16 *>(bf16_output);
   const size_t elements = static_cast<size_t>(rows) * width;
-  const bool vectors = elements > 65536 && width % 8 == 0 && output_width % 8 == 0 && first_column % 8 == 0 &&
+  const bool vectors = elements > 512 * 1024 && width % 8 == 0 && output_width % 8 == 0 && first_column % 8 == 0 &&
                        reinterpret_cast<uintptr_t>(partial) % 16 == 0 &&
                        reinterpret_cast<uintptr_t>(output) % 16 == 0 && elements / 8 < 0x7FFFFF00U;
   if (vectors) {

@@ -23,7 +23,8 @@ struct LinearPlan {
   int rows{0};
   int input_width{0};
   int output_width{0};
-  int padded_rows{0};       // UMMA N: 32, 64, 128, 192 or 256
+  int padded_rows{0};       // UMMA N: the rows rounded up to 32 (gated plans: 32, 64, 128, 192, 256;
+                            // CTA pairs: to 16 or 32, see pair_tile_rows)
   int tile_width{0};        // output features per tile: 256 (CTA pairs), 128 in a gated plan
   int tiles{0};             // output-feature tiles
   int k_blocks{0};          // 128-byte K blocks
