@@ -896,11 +896,11 @@ int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_we
   return 0;
 }
 
-int retarget_linear_plan(LinearPlan *plan, const void *input, int rows) {
+int retarget_linear_plan(LinearPlan *plan, const void *input, int rows, int requested_splits) {
   LinearPlan result{};
   result.weight_map = plan->weight_map;
   if (rows <= 0 || (reinterpret_cast<uintptr_t>(input) & 15U) != 0 ||
-      !schedule_plain(&result, rows, plan->input_width, plan->output_width, 0,
+      !schedule_plain(&result, rows, plan->input_width, plan->output_width, requested_splits,
                       plan->element_bytes)) {
     return -1;
   }

@@ -54,7 +54,7 @@ int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_we
 
 // The same plan for another number of rows of another input of the same width: the schedule and
 // the input map are made again, the weight map stays.
-int retarget_linear_plan(LinearPlan *plan, const void *input, int rows);
+int retarget_linear_plan(LinearPlan *plan, const void *input, int rows, int requested_splits = 0);
 
 // The gate_up linear with GeGLU in its epilogue. `fp8_weight` is [2 * gated_width, input_width]
 // with the gate rows first; gated_width must be a multiple of 64.

@@ -449,18 +449,15 @@ __global__ void prefill_gather_kernel(PrefillGatherArguments a) {
   }
 }
 
-__global__ void prefill_last_rows_kernel(const uint4 *source, const int *rows, const int *slots,
-                                         int vectors, uint4 *destination, uint4 *table) {
+__global__ void copy_rows_kernel(const uint4 *source, const int *from, uint4 *destination,
+                                 const int *to, int vectors) {
   grid_dependency_launch();
+  const int index = static_cast<int>(blockIdx.x);
+  const long long first = static_cast<long long>(from != nullptr ? from[index] : index) * vectors;
+  const long long last = static_cast<long long>(to != nullptr ? to[index] : index) * vectors;
   grid_dependency_wait();
-  const long long from = static_cast<long long>(rows[blockIdx.x]) * vectors;
-  const long long to = static_cast<long long>(blockIdx.x) * vectors;
-  const long long slot = static_cast<long long>(slots[blockIdx.x]) * vectors;
-  for (int vector = static_cast<int>(threadIdx.x); vector < vectors; vector += blockDim.x) {
-    const uint4 value = source[from + vector];
-    destination[to + vector] = value;
-    table[slot + vector] = value;
-  }
+  for (int vector = static_cast<int>(threadIdx.x); vector < vectors; vector += blockDim.x)
+    destination[last + vector] = source[first + vector];
 }
 
 bool encode_rows(CUtensorMap *map, const void *base, long long rows, int columns) {
@@ -554,16 +551,13 @@ int launch_prefill_gather(const PrefillGatherArguments &a, cudaStream_t stream) 
              : -11;
 }
 
-int launch_prefill_last_rows(const void *source, const int *rows, const int *slots, int count,
-                             int width, void *destination, void *table, cudaStream_t stream) {
-  if (source == nullptr || rows == nullptr || slots == nullptr || destination == nullptr ||
-      table == nullptr || count <= 0 || width <= 0 || width % 8 != 0) {
+int launch_copy_rows(const void *source, const int *from, void *destination, const int *to,
+                     int count, int width, cudaStream_t stream) {
+  if (source == nullptr || destination == nullptr || count <= 0 || width <= 0 || width % 8 != 0)
     return -1;
-  }
-  return launch_chained(prefill_last_rows_kernel, dim3(static_cast<unsigned>(count)), dim3(256), 0,
-                        stream, false, static_cast<const uint4 *>(source), rows, slots, width / 8,
-                        static_cast<uint4 *>(destination), static_cast<uint4 *>(table)) ==
-                 cudaSuccess
+  return launch_chained(copy_rows_kernel, dim3(static_cast<unsigned>(count)), dim3(256), 0, stream,
+                        false, static_cast<const uint4 *>(source), from,
+                        static_cast<uint4 *>(destination), to, width / 8) == cudaSuccess
              ? 0
              : -11;
 }

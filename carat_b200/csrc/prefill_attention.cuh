@@ -81,9 +81,9 @@ struct PrefillGatherArguments {
 };
 int launch_prefill_gather(const PrefillGatherArguments &arguments, cudaStream_t stream);
 
-// destination[i] = source[rows[i]], and again to table[slots[i]]: the last rows of the prompts that
-// became resident, for the LM head and for the drafter. Rows of `width` bf16 values.
-int launch_prefill_last_rows(const void *source, const int *rows, const int *slots, int count,
-                             int width, void *destination, void *table, cudaStream_t stream);
+// destination[to[i]] = source[from[i]] (null: i), rows of `width` bf16 values. Picks the last rows of
+// the prompts that become resident, and hands their final hidden rows to the drafter's table.
+int launch_copy_rows(const void *source, const int *from, void *destination, const int *to,
+                     int count, int width, cudaStream_t stream);
 
 } // namespace carat_b200

@@ -402,10 +402,13 @@ int launch_qkv_post(const QkvPostArguments &a, cudaStream_t stream) {
 
 int launch_prefill_qkv_post(const PrefillQkvArguments &a, cudaStream_t stream) {
   if (a.packed == nullptr || a.query_norm == nullptr || a.key_norm == nullptr ||
-      a.cosine == nullptr || a.sine == nullptr || a.queries == nullptr || a.positions == nullptr ||
-      a.cache_slots == nullptr || a.key_cache == nullptr || a.value_cache == nullptr ||
+      a.cosine == nullptr || a.sine == nullptr || a.positions == nullptr ||
+      (a.query_heads > 0 && a.queries == nullptr) ||
+      (a.kv_heads > 0 &&
+       (a.cache_slots == nullptr || a.key_cache == nullptr || a.value_cache == nullptr)) ||
       (a.staged_rows != nullptr && (a.staged_keys == nullptr || a.staged_values == nullptr)) ||
-      a.rows <= 0 || a.query_heads <= 0 || a.kv_heads <= 0 || a.capacity <= 0 ||
+      a.rows <= 0 || a.query_heads < 0 || a.kv_heads < 0 || a.query_heads + a.kv_heads == 0 ||
+      a.capacity <= 0 ||
       a.slot_stride % 8 != 0 || a.head_stride % 8 != 0 ||
       !aligned16(a.packed, a.query_norm, a.key_norm, a.cosine, a.sine, a.queries, a.key_cache,
                  a.value_cache, a.staged_keys, a.staged_values)) {

@@ -48,6 +48,7 @@ struct QkvPostArguments {
 int launch_qkv_post(const QkvPostArguments &arguments, cudaStream_t stream);
 
 // The same for a prefill step: packed rows of several requests, position and owner per row.
+// Either may be absent (query_heads or kv_heads 0): the packed rows then hold the other part only.
 // Q goes to [rows, query_heads, head_dim]. A row's K and V go to the staging buffer
 // [staging rows][kv_heads * head_dim] when staged_rows is given (sliding layers), and to its slot's
 // cache at position % capacity when cache_slots[row] >= 0.

@@ -228,10 +228,13 @@ struct carat_b200_runner {
   struct PrefillLayer {
     LinearPlan qkv, o, gate_up, down;   // only their weight maps are used
   };
+  // The last layer makes K and V of every row but Q and all that follows of a prompt's last row
+  // only, so its fused projection is planned as its two parts.
+  LinearPlan q_last_query, q_last_key_value;
   std::vector<PrefillLayer> q_layers;
   DeviceBuffer q_hidden_a, q_hidden_b, q_residual, q_normed, q_pre_mlp, q_activated, q_packed,
-      q_queries, q_attention, q_projected, q_gate_up, q_final, q_partials, q_staged, q_inputs,
-      q_last_rows;
+      q_queries, q_attention, q_projected, q_gate_up, q_partials, q_staged, q_inputs,
+      q_last_rows, q_last_normed, q_last_hidden, q_key_value;
   PinnedBuffer q_host_inputs;
   size_t q_staged_value_offset{0};
   int q_staging_rows{0};
@@ -1422,7 +1425,8 @@ void prefill_step(Runner &runner, const int *tokens, int requests, int depth, co
 
 // Where the pieces of a packed prefill step's input block are, in ints.
 struct PackedInputs {
-  int tokens, positions, sliding_slots, global_slots, staged_rows, last_rows, last_slots;
+  int tokens, positions, sliding_slots, global_slots, staged_rows, last_rows, last_slots,
+      last_positions;
   int segments, tiles, total;
   PackedInputs(int rows, int batch, int most_tiles) {
     int at = 0;
@@ -1438,6 +1442,7 @@ struct PackedInputs {
     staged_rows = take(rows);
     last_rows = take(batch);
     last_slots = take(batch);
+    last_positions = take(batch);
     segments = take(batch * static_cast<int>(sizeof(PrefillSegment) / sizeof(int)));
     tiles = take(most_tiles * static_cast<int>(sizeof(PrefillTile) / sizeof(int)));
     total = at;
@@ -1452,8 +1457,8 @@ int packed_prefill_tiles(const Runner &runner) {
     const int tokens = 128 / (layer.shape.query_heads / layer.shape.kv_heads);
     most += packed_prefill_rows / tokens + runner.batch;
   }
-  // One list per distinct tile size; layers share them.
-  return std::min(most, 8 * (packed_prefill_rows + runner.batch));
+  // One list per distinct tile size, which layers share, and one of single rows.
+  return std::min(most, 8 * (packed_prefill_rows + runner.batch)) + runner.batch;
 }
 
 bool packed_prefill_takes(const Runner &runner) {
@@ -1494,15 +1499,18 @@ void prepare_packed_prefill(Runner &runner) {
       widest_staged = std::max(widest_staged, static_cast<size_t>(layer.kv_width()));
   }
   for (DeviceBuffer *buffer : {&runner.q_hidden_a, &runner.q_hidden_b, &runner.q_residual,
-                               &runner.q_normed, &runner.q_pre_mlp, &runner.q_projected,
-                               &runner.q_final})
+                               &runner.q_normed, &runner.q_pre_mlp, &runner.q_projected})
     buffer->allocate(row_hidden);
   runner.q_activated.allocate(rows * config.intermediate_size * 2);
   runner.q_packed.allocate(rows * widest_packed * 2);
   runner.q_queries.allocate(rows * widest_query * 2, true);
   runner.q_attention.allocate(rows * widest_query * 2);
   runner.q_gate_up.allocate(rows * 2 * config.intermediate_size * 2);
-  runner.q_last_rows.allocate(static_cast<size_t>(runner.batch) * config.hidden_size * 2);
+  for (DeviceBuffer *buffer : {&runner.q_last_rows, &runner.q_last_normed, &runner.q_last_hidden})
+    buffer->allocate(static_cast<size_t>(runner.batch) * config.hidden_size * 2);
+  const LayerState &last_layer = runner.layers.back();
+  const int last_key_value = last_layer.packed_width() - last_layer.query_width();
+  runner.q_key_value.allocate(rows * last_key_value * 2);
   // Every segment brings at most a window and two partial tiles beside its own rows.
   const int window_rows = std::min(config.sliding_window, runner.maximum_context);
   runner.q_staging_rows =
@@ -1538,6 +1546,19 @@ void prepare_packed_prefill(Runner &runner) {
     entry.down = plan(runner.q_activated.get(), weights.down, config.intermediate_size,
                       config.hidden_size);
     runner.q_layers.push_back(entry);
+    if (index + 1 == runner.layers.size()) {
+      runner.q_last_query = plan_bf16_linear(runner.q_last_normed.get(), weights.qkv, 1,
+                                             config.hidden_size, layer.query_width(), 0);
+      partial_bytes = std::max(
+          partial_bytes, linear_partial_bytes_for(std::min(runner.batch, maximum_rows),
+                                                  config.hidden_size, layer.query_width(), 2));
+      // Not cut: its few tiles are enough for a step's rows, and its sums go straight to bf16.
+      runner.q_last_key_value = plan_bf16_linear(
+          runner.q_normed.get(),
+          static_cast<const unsigned char *>(weights.qkv) +
+              static_cast<size_t>(layer.query_width()) * config.hidden_size * 2,
+          packed_prefill_rows, config.hidden_size, last_key_value, 1, packed_prefill_rows);
+    }
   }
   runner.q_partials.allocate(std::max<size_t>(partial_bytes, 256));
 }
@@ -1547,7 +1568,8 @@ void prepare_packed_prefill(Runner &runner) {
 // Rows of different segments only share the linears, and every sum's order depends on the widths
 // and on a row's position alone, so a row's result does not depend on the step it is in.
 // `complete[s]` marks segments whose last row ends a prompt: its final-normed hidden row goes to the
-// slot's hand-off row and the bf16 LM head predicts its next token into predictions[s].
+// slot's hand-off row and the bf16 LM head predicts its next token into predictions[s]. Only those
+// rows go through the last layer beyond its K and V (six layers, 777 rows: 5.4 ms with all rows).
 void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
                        std::vector<PrefillSegment> &segments, const std::vector<bool> &complete,
                        std::vector<int> &predictions) {
@@ -1583,6 +1605,7 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
     if (complete[index]) {
       host[layout.last_rows + last_count] = row - 1;
       host[layout.last_slots + last_count] = segment.slot;
+      host[layout.last_positions + last_count] = segment.first + segment.count - 1;
       ++last_count;
     }
   }
@@ -1640,8 +1663,28 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
     return lists.back();
   };
   std::vector<TileList> layer_tiles;
-  for (const LayerState &layer : runner.layers)
-    layer_tiles.push_back(tiles_for(layer));
+  for (int index = 0; index + 1 < config.layer_count; ++index)
+    layer_tiles.push_back(tiles_for(runner.layers[static_cast<size_t>(index)]));
+  {
+    // The last layer: the prompts' last rows, packed in the order of last_rows, one a tile.
+    const LayerState &layer = runner.layers.back();
+    const bool global = layer.shape.global_attention != 0;
+    TileList list{1, global, layer.capacity, layer.shape.kv_heads, tile_count, 0};
+    for (size_t index = 0; index < segments.size(); ++index) {
+      if (!complete[index])
+        continue;
+      if (tile_count >= most_tiles)
+        throw Failure{"invalid batched chunk prefill shape"};
+      const PrefillSegment &segment = segments[index];
+      PrefillTile &tile = host_tiles[tile_count++];
+      tile.row = list.count++;
+      tile.tokens = 1;
+      tile.position = segment.first + segment.count - 1;
+      tile.key_base = global ? segment.slot * layer.shape.kv_heads * layer.capacity
+                             : segment.stage_row - segment.origin;
+    }
+    layer_tiles.push_back(list);
+  }
   require_cuda(cudaMemcpyAsync(runner.q_inputs.get(), host,
                                sizeof(int) * static_cast<size_t>(layout.tiles) +
                                    sizeof(PrefillTile) * static_cast<size_t>(tile_count),
@@ -1658,9 +1701,11 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
   // ---- plans: schedules and input maps depend on the widths and the row count only, so layers
   // share them and bring their weight maps.
   std::vector<std::pair<const void *, LinearPlan>> shared;
-  const auto plan_for = [&](const LinearPlan &layer_plan, const void *input) {
+  const auto plan_for = [&](const LinearPlan &layer_plan, const void *input, int plan_rows,
+                            int splits = 0) {
     for (const auto &entry : shared) {
-      if (entry.first == input && entry.second.input_width == layer_plan.input_width &&
+      if (entry.first == input && entry.second.rows == plan_rows &&
+          entry.second.input_width == layer_plan.input_width &&
           entry.second.output_width == layer_plan.output_width) {
         LinearPlan plan = entry.second;
         plan.weight_map = layer_plan.weight_map;
@@ -1668,7 +1713,7 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
       }
     }
     LinearPlan plan = layer_plan;
-    if (retarget_linear_plan(&plan, input, rows) != 0)
+    if (retarget_linear_plan(&plan, input, plan_rows, splits) != 0)
       throw Failure{"invalid BF16 linear shape"};
     shared.emplace_back(input, plan);
     return plan;
@@ -1699,33 +1744,63 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
                                          epsilon, nullptr, 0, stream),
                  "embedding and input norm");
   runner.launches += 1;
+  // A linear whose sums the kernel after it does not take in pieces.
+  const auto finished = [&](const LinearPlan &plan, void *output, int plan_rows, int width) {
+    const PartialSource source = linear(plan, output);
+    if (source.splits > 0) {
+      require_launch(launch_quant(nullptr, partials, source.splits, nullptr, 1, rows_only(output),
+                                  plan_rows, width, stream),
+                     "BF16 linear rows");
+      runner.launches += 1;
+    }
+  };
+  const auto post_process = [&](const LayerState &layer, const void *packed, int post_rows,
+                                const int *positions, int query_heads, int kv_heads) {
+    const RopeTable &rope = *runner.rope_tables[static_cast<size_t>(layer.rope)];
+    const bool global = layer.shape.global_attention != 0;
+    PrefillQkvArguments post{};
+    post.packed = packed;
+    post.query_norm = layer.weights.q_norm;
+    post.key_norm = layer.weights.k_norm;
+    post.cosine = rope.cosine.get();
+    post.sine = rope.sine.get();
+    post.queries = runner.q_queries.get();
+    post.positions = positions;
+    post.cache_slots = device + (global ? layout.global_slots : layout.sliding_slots);
+    post.staged_rows = global || kv_heads == 0 ? nullptr : device + layout.staged_rows;
+    post.staged_keys = global ? nullptr : runner.q_staged.get();
+    post.staged_values =
+        global ? nullptr : runner.q_staged.get<unsigned char>() + runner.q_staged_value_offset;
+    post.key_cache = layer.keys();
+    post.value_cache = layer.values();
+    post.slot_stride = layer.slot_stride;
+    post.head_stride = layer.head_stride;
+    post.rows = post_rows;
+    post.capacity = layer.capacity;
+    post.query_heads = query_heads;
+    post.kv_heads = kv_heads;
+    post.head_dim = layer.shape.head_dim;
+    post.key_equals_value = layer.shape.key_equals_value;
+    post.max_positions = runner.maximum_context;
+    post.epsilon = epsilon;
+    require_launch(launch_prefill_qkv_post(post, stream), "QKV post-processing");
+    runner.launches += 1;
+  };
   for (int index = 0; index < config.layer_count; ++index) {
     const LayerState &layer = runner.layers[static_cast<size_t>(index)];
     const Runner::PrefillLayer &plans = runner.q_layers[static_cast<size_t>(index)];
     const auto &shape = layer.shape;
     const auto &w = layer.weights;
-    const RopeTable &rope = *runner.rope_tables[static_cast<size_t>(layer.rope)];
     const bool global = shape.global_attention != 0;
-    const LinearPlan qkv = plan_for(plans.qkv, runner.q_normed.get());
-    const PartialSource packed = linear(qkv, runner.q_packed.get());
-    if (packed.splits > 0) {
-      // Few output features: the K pieces are summed to bf16 rows for the post-processing.
-      require_launch(launch_quant(nullptr, partials, packed.splits, nullptr, 1,
-                                  rows_only(runner.q_packed.get()), rows, layer.packed_width(),
-                                  stream),
-                     "QKV rows");
-      runner.launches += 1;
-    }
-    void *staged_keys = runner.q_staged.get();
-    void *staged_values = runner.q_staged.get<unsigned char>() + runner.q_staged_value_offset;
+    const bool last = index + 1 == config.layer_count;
     if (!global) {
       PrefillGatherArguments gather{};
       gather.segments = reinterpret_cast<const PrefillSegment *>(device + layout.segments);
       gather.segment_count = static_cast<int>(segments.size());
       gather.key_cache = layer.keys();
       gather.value_cache = layer.values();
-      gather.staged_keys = staged_keys;
-      gather.staged_values = staged_values;
+      gather.staged_keys = runner.q_staged.get();
+      gather.staged_values = runner.q_staged.get<unsigned char>() + runner.q_staged_value_offset;
       gather.slot_stride = layer.slot_stride;
       gather.head_stride = layer.head_stride;
       gather.capacity = layer.capacity;
@@ -1735,38 +1810,43 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
       require_launch(launch_prefill_gather(gather, stream), "prefill ring rows");
       runner.launches += 1;
     }
-    PrefillQkvArguments post{};
-    post.packed = runner.q_packed.get();
-    post.query_norm = w.q_norm;
-    post.key_norm = w.k_norm;
-    post.cosine = rope.cosine.get();
-    post.sine = rope.sine.get();
-    post.queries = runner.q_queries.get();
-    post.positions = device + layout.positions;
-    post.cache_slots = device + (global ? layout.global_slots : layout.sliding_slots);
-    post.staged_rows = global ? nullptr : device + layout.staged_rows;
-    post.staged_keys = global ? nullptr : staged_keys;
-    post.staged_values = global ? nullptr : staged_values;
-    post.key_cache = layer.keys();
-    post.value_cache = layer.values();
-    post.slot_stride = layer.slot_stride;
-    post.head_stride = layer.head_stride;
-    post.rows = rows;
-    post.capacity = layer.capacity;
-    post.query_heads = shape.query_heads;
-    post.kv_heads = shape.kv_heads;
-    post.head_dim = shape.head_dim;
-    post.key_equals_value = shape.key_equals_value;
-    post.max_positions = runner.maximum_context;
-    post.epsilon = epsilon;
-    require_launch(launch_prefill_qkv_post(post, stream), "QKV post-processing");
-    runner.launches += 1;
+    // The last layer leaves K and V of every row in the cache; nothing else of it is used but the
+    // last rows of prompts that end in this step.
+    const int live = last ? last_count : rows;
+    const void *residual = current;
+    if (!last) {
+      finished(plan_for(plans.qkv, runner.q_normed.get(), rows), runner.q_packed.get(), rows,
+               layer.packed_width());
+      post_process(layer, runner.q_packed.get(), rows, device + layout.positions,
+                   shape.query_heads, shape.kv_heads);
+    } else {
+      finished(plan_for(runner.q_last_key_value, runner.q_normed.get(), rows, 1),
+               runner.q_key_value.get(), rows, layer.packed_width() - layer.query_width());
+      post_process(layer, runner.q_key_value.get(), rows, device + layout.positions, 0,
+                   shape.kv_heads);
+      if (live == 0)
+        break;
+      require_launch(launch_copy_rows(runner.q_normed.get(), device + layout.last_rows,
+                                      runner.q_last_normed.get(), nullptr, live, hidden, stream),
+                     "last rows");
+      require_launch(launch_copy_rows(current, device + layout.last_rows,
+                                      runner.q_last_hidden.get(), nullptr, live, hidden, stream),
+                     "last rows");
+      runner.launches += 2;
+      residual = runner.q_last_hidden.get();
+      finished(plan_for(runner.q_last_query, runner.q_last_normed.get(), live),
+               runner.q_packed.get(), live, layer.query_width());
+      post_process(layer, runner.q_packed.get(), live, device + layout.last_positions,
+                   shape.query_heads, 0);
+    }
 
     const TileList &list = layer_tiles[static_cast<size_t>(index)];
+    void *staged_values =
+        runner.q_staged.get<unsigned char>() + runner.q_staged_value_offset;
     PrefillAttentionMaps maps;
     const int status = make_prefill_attention_maps(
         &maps, runner.q_queries.get(), packed_prefill_rows, shape.query_heads, shape.kv_heads,
-        shape.head_dim, global ? layer.keys() : staged_keys,
+        shape.head_dim, global ? layer.keys() : runner.q_staged.get(),
         global ? layer.values() : staged_values,
         global ? static_cast<long long>(runner.batch) * shape.kv_heads * layer.capacity
                : runner.q_staging_rows,
@@ -1788,15 +1868,15 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
     require_launch(launch_prefill_attention(maps, attention, stream), "prefill attention");
     runner.launches += 1;
 
-    const PartialSource o_source =
-        linear(plan_for(plans.o, runner.q_attention.get()), runner.q_projected.get());
+    const PartialSource o_source = linear(plan_for(plans.o, runner.q_attention.get(), live),
+                                          runner.q_projected.get());
     require_launch(launch_post_attention_norms_quant(
-                       runner.q_projected.get(), o_source, w.post_attention_norm, current,
+                       runner.q_projected.get(), o_source, w.post_attention_norm, residual,
                        w.pre_mlp_norm, runner.q_residual.get(), rows_only(runner.q_pre_mlp.get()),
-                       rows, hidden, epsilon, stream),
+                       live, hidden, epsilon, stream),
                    "post-attention norms");
     runner.launches += 1;
-    const LinearPlan gate_up = plan_for(plans.gate_up, runner.q_pre_mlp.get());
+    const LinearPlan gate_up = plan_for(plans.gate_up, runner.q_pre_mlp.get(), live);
     TailSource tail{};
     if (gate_up.splits == 1 && gate_up.tail_tiles > 0 &&
         gate_up.tail_columns() <= config.intermediate_size) {
@@ -1809,29 +1889,21 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
                         2 * config.intermediate_size - gate_up.tail_columns(),
                         gate_up.tail_columns(), unit, unit};
     } else {
-      const PartialSource up = linear(gate_up, runner.q_gate_up.get());
-      if (up.splits > 0) {
-        require_launch(launch_quant(nullptr, partials, up.splits, nullptr, 1,
-                                    rows_only(runner.q_gate_up.get()), rows,
-                                    2 * config.intermediate_size, stream),
-                       "gate_up rows");
-        runner.launches += 1;
-      }
+      finished(gate_up, runner.q_gate_up.get(), live, 2 * config.intermediate_size);
     }
     require_launch(launch_geglu_quant(runner.q_gate_up.get(), tail,
-                                      rows_only(runner.q_activated.get()), rows,
+                                      rows_only(runner.q_activated.get()), live,
                                       config.intermediate_size, stream),
                    "GeGLU");
     runner.launches += 1;
-    const PartialSource down_source =
-        linear(plan_for(plans.down, runner.q_activated.get()), runner.q_projected.get());
-    const bool last = index + 1 == config.layer_count;
+    const PartialSource down_source = linear(
+        plan_for(plans.down, runner.q_activated.get(), live), runner.q_projected.get());
     const void *next_norm = last ? runner.weights.final_norm
                                  : runner.layers[static_cast<size_t>(index) + 1].weights.input_norm;
     require_launch(launch_layer_output_norm_quant(
                        runner.q_projected.get(), down_source, w.post_mlp_norm,
                        runner.q_residual.get(), w.scalar, other, next_norm,
-                       last ? runner.q_final.get() : runner.q_normed.get(), QuantTarget{}, rows,
+                       last ? runner.q_last_rows.get() : runner.q_normed.get(), QuantTarget{}, live,
                        hidden, epsilon, stream),
                    "layer output");
     runner.launches += 1;
@@ -1839,10 +1911,8 @@ void prefill_rows_step(Runner &runner, const std::vector<int> &tokens,
   }
   int *host_results = runner.host_results.get<int>();
   if (last_count > 0) {
-    require_launch(launch_prefill_last_rows(runner.q_final.get(), device + layout.last_rows,
-                                            device + layout.last_slots, last_count, hidden,
-                                            runner.q_last_rows.get(), runner.hidden_by_slot.get(),
-                                            stream),
+    require_launch(launch_copy_rows(runner.q_last_rows.get(), nullptr, runner.hidden_by_slot.get(),
+                                    device + layout.last_slots, last_count, hidden, stream),
                    "prefill hand-off rows");
     const LinearPlan head =
         plan_bf16_linear(runner.q_last_rows.get(), runner.weights.token_embedding, last_count,
@@ -2433,7 +2503,8 @@ extern "C" int carat_b200_runner_prefill_slots_chunks(
         std::vector<bool> complete;
         std::vector<int> owners;
         while (request < requests &&
-               static_cast<int>(step_tokens.size()) < packed_prefill_rows) {
+               static_cast<int>(step_tokens.size()) < packed_prefill_rows &&
+               static_cast<int>(segments.size()) < maximum_rows) {
           const size_t r = static_cast<size_t>(request);
           const int count = std::min(end[r] - at[r], packed_prefill_rows -
                                                          static_cast<int>(step_tokens.size()));
