@@ -812,7 +812,9 @@ int launch_planned(const LinearPlan &plan, const KernelArguments &arguments, cud
 // start and end cost two cluster barriers) and a tile is long enough to hide those: bf16
 // 5376 -> 43008 at 256 rows 103 us against 119, 192 rows 85 against 91, 128 rows 79 against 79,
 // 24 rows 70 against 68; e4m3 256 rows 59 to 64 against 67 to 73, 192 rows 54 against 54; but
-// bf16 1024 -> 262144 (16 blocks of K) 240 against 235 at 256 rows.
+// bf16 1024 -> 262144 (16 blocks of K) 240 against 235 at 256 rows. A launch long enough to forget
+// its start (the LM head: eight rounds of tiles and more) has them from 97 rows on: e4m3
+// 5376 -> 262144 120 rows 225 against 236, 160 rows 242 against 256, but 72 rows 216 against 216.
 bool schedule_plain(LinearPlan *plan, int rows, int input_width, int output_width,
                     int requested_splits, int element_bytes) {
   schedule_linear(plan, rows, input_width, output_width, requested_splits, element_bytes);
@@ -820,7 +822,7 @@ bool schedule_plain(LinearPlan *plan, int rows, int input_width, int output_widt
   if (rows > 256)
     return schedule_pairs(plan);
   if (plan->splits == 1 && plan->tiles >= plan->ctas / 2 && plan->k_blocks >= 32 &&
-      rows > (element_bytes == 2 ? 160 : 192)) {
+      (rows > (element_bytes == 2 ? 160 : 192) || (rows > 96 && plan->tiles >= 8 * plan->ctas))) {
     schedule_pairs(plan);   // keeps the plan when it cannot
   }
   return true;
