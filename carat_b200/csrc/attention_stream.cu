@@ -438,48 +438,49 @@ scores_stream_kernel(const __grid_constant__ CUtensorMap key_map,
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint64_t key_desc = ptx::umma_desc_k_major_sw128(ring);
-      const uint32_t desc_high = static_cast<uint32_t>(key_desc >> 32);
-      const uint32_t key_low = static_cast<uint32_t>(key_desc);
-      const uint32_t query_low = static_cast<uint32_t>(ptx::umma_desc_k_major_sw128(query_tiles));
-      Cursor<stages> cursor;
-      uint32_t accumulator = 0;
-      uint32_t accumulator_phase = 0;
-      bool healthy = true;
-      uint32_t local = 0;
-      for (int ordinal = 0; ordinal < schedule.count && healthy; ++ordinal) {
-        const StreamItem item = cached_item(a, schedule, ordinal);
-        if (item.empty())
-          continue;
-        if (!ptx::mbarrier_wait_checked(query_full_bar, local & 1U, abort_flag, args.device_error, 42)) {
-          healthy = false;
+    // The whole warp walks the loop in lockstep and one elected lane issues: the loop state stays
+    // warp-uniform (descriptor and ring arithmetic on the uniform datapath), where a single-lane
+    // loop competed with the epilogue warps for issue slots at every step.
+    const uint64_t key_desc = ptx::umma_desc_k_major_sw128(ring);
+    const uint32_t desc_high = static_cast<uint32_t>(key_desc >> 32);
+    const uint32_t key_low = static_cast<uint32_t>(key_desc);
+    const uint32_t query_low = static_cast<uint32_t>(ptx::umma_desc_k_major_sw128(query_tiles));
+    Cursor<stages> cursor;
+    uint32_t accumulator = 0;
+    uint32_t accumulator_phase = 0;
+    bool healthy = true;
+    uint32_t local = 0;
+    const auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+      const bool ready = ptx::mbarrier_wait_checked(bar, parity, abort_flag, args.device_error, code);
+      if (__all_sync(0xFFFFFFFFU, ready ? 1 : 0) == 0)
+        healthy = false;
+      return healthy;
+    };
+    for (int ordinal = 0; ordinal < schedule.count && healthy; ++ordinal) {
+      const StreamItem item = cached_item(a, schedule, ordinal);
+      if (item.empty())
+        continue;
+      if (!wait(query_full_bar, local & 1U, 42))
+        break;
+      ++local;
+      const int tiles = (item.proposals > 0 ? 1 : 0) +
+                        (item.rows_here + stream_tile_keys - 1) / stream_tile_keys;
+      for (int tile = 0; tile < tiles && healthy; ++tile) {
+        if (!wait(acc_empty_bar + 8U * accumulator, accumulator_phase ^ 1U, 43))
           break;
-        }
-        ++local;
-        const int tiles = (item.proposals > 0 ? 1 : 0) +
-                          (item.rows_here + stream_tile_keys - 1) / stream_tile_keys;
-        for (int tile = 0; tile < tiles && healthy; ++tile) {
-          if (!ptx::mbarrier_wait_checked(acc_empty_bar + 8U * accumulator, accumulator_phase ^ 1U, abort_flag,
-                            args.device_error, 43)) {
-            healthy = false;
-            break;
-          }
-          ptx::tcgen05_fence_after_thread_sync();
-          const uint32_t tmem_scores = tmem_base + accumulator * padded_rows;
+        ptx::tcgen05_fence_after_thread_sync();
+        const uint32_t tmem_scores = tmem_base + accumulator * padded_rows;
 #pragma unroll
-          for (int pair = 0; pair < subtiles / 2; ++pair) {
-            if (!ptx::mbarrier_wait_checked(full_bar + 8U * cursor.stage, cursor.phase, abort_flag,
-                              args.device_error, 44)) {
-              healthy = false;
-              break;
-            }
-            ptx::tcgen05_fence_after_thread_sync();
+        for (int pair = 0; pair < subtiles / 2; ++pair) {
+          if (!wait(full_bar + 8U * cursor.stage, cursor.phase, 44))
+            break;
+          ptx::tcgen05_fence_after_thread_sync();
+          const uint32_t stage_low = key_low + cursor.stage * (stream_stage_bytes >> 4);
+          if (ptx::elect_one()) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
               const int sub = pair * 2 + half;
-              const uint32_t a_low = key_low + cursor.stage * (stream_stage_bytes >> 4) +
-                                     half * (stream_subtile_bytes >> 4);
+              const uint32_t a_low = stage_low + half * (stream_subtile_bytes >> 4);
               const uint32_t b_low = query_low + sub * ((padded_rows * 128) >> 4);
 #pragma unroll
               for (int step = 0; step < 4; ++step)
@@ -488,17 +489,20 @@ scores_stream_kernel(const __grid_constant__ CUtensorMap key_map,
                                            (sub > 0 || step > 0) ? 1U : 0U);
             }
             ptx::tcgen05_commit(empty_bar + 8U * cursor.stage);
-            cursor.advance();
           }
-          if (healthy)
-            ptx::tcgen05_commit(acc_full_bar + 8U * accumulator);
-          accumulator ^= 1U;
-          if (accumulator == 0)
-            accumulator_phase ^= 1U;
+          __syncwarp();
+          cursor.advance();
         }
-        if (healthy)
-          ptx::tcgen05_commit(query_free_bar);
+        if (healthy && ptx::elect_one())
+          ptx::tcgen05_commit(acc_full_bar + 8U * accumulator);
+        __syncwarp();
+        accumulator ^= 1U;
+        if (accumulator == 0)
+          accumulator_phase ^= 1U;
       }
+      if (healthy && ptx::elect_one())
+        ptx::tcgen05_commit(query_free_bar);
+      __syncwarp();
     }
   } else {
     const int epilogue_warp = warp - 2;
@@ -810,74 +814,72 @@ values_stream_kernel(const __grid_constant__ CUtensorMap value_map,
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint64_t value_desc = ptx::umma_desc_mn_major_sw128(ring, Shape::value_box_bytes);
-      const uint32_t desc_high = static_cast<uint32_t>(value_desc >> 32);
-      const uint32_t value_low = static_cast<uint32_t>(value_desc);
-      const uint32_t probability_low =
-          static_cast<uint32_t>(ptx::umma_desc_k_major_sw128(probability_ring));
-      Cursor<stages> cursor;
-      Cursor<probability_boxes> probability_cursor;
-      bool healthy = true;
-      uint32_t local = 0;
-      for (int ordinal = 0; ordinal < schedule.count && healthy; ++ordinal) {
-        const StreamItem item = cached_item(a, schedule, ordinal);
-        if (item.empty())
-          continue;
-        const uint32_t buffer = output_buffers == 2 ? (local & 1U) : 0U;
-        const uint32_t use = output_buffers == 2 ? (local >> 1) : local;
-        ++local;
-        if (!ptx::mbarrier_wait_checked(o_empty_bar + 8U * buffer, (use & 1U) ^ 1U, abort_flag,
-                          args.device_error, 51)) {
-          healthy = false;
+    // Warp-uniform loop, one elected lane issues (as in the scores kernel).
+    const uint64_t value_desc = ptx::umma_desc_mn_major_sw128(ring, Shape::value_box_bytes);
+    const uint32_t desc_high = static_cast<uint32_t>(value_desc >> 32);
+    const uint32_t value_low = static_cast<uint32_t>(value_desc);
+    const uint32_t probability_low =
+        static_cast<uint32_t>(ptx::umma_desc_k_major_sw128(probability_ring));
+    Cursor<stages> cursor;
+    Cursor<probability_boxes> probability_cursor;
+    bool healthy = true;
+    uint32_t local = 0;
+    const auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+      const bool ready = ptx::mbarrier_wait_checked(bar, parity, abort_flag, args.device_error, code);
+      if (__all_sync(0xFFFFFFFFU, ready ? 1 : 0) == 0)
+        healthy = false;
+      return healthy;
+    };
+    for (int ordinal = 0; ordinal < schedule.count && healthy; ++ordinal) {
+      const StreamItem item = cached_item(a, schedule, ordinal);
+      if (item.empty())
+        continue;
+      const uint32_t buffer = output_buffers == 2 ? (local & 1U) : 0U;
+      const uint32_t use = output_buffers == 2 ? (local >> 1) : local;
+      ++local;
+      if (!wait(o_empty_bar + 8U * buffer, (use & 1U) ^ 1U, 51))
+        break;
+      ptx::tcgen05_fence_after_thread_sync();
+      const uint32_t tmem_output = tmem_base + buffer * Shape::output_columns;
+      uint32_t accumulate = 0;
+      if (item.proposals > 0) {
+        if (!wait(p_full_bar + 8U * probability_cursor.stage, probability_cursor.phase, 52) ||
+            !wait(full_bar + 8U * cursor.stage, cursor.phase, 53))
           break;
-        }
         ptx::tcgen05_fence_after_thread_sync();
-        const uint32_t tmem_output = tmem_base + buffer * Shape::output_columns;
-        uint32_t accumulate = 0;
-        if (item.proposals > 0) {
-          if (!ptx::mbarrier_wait_checked(p_full_bar + 8U * probability_cursor.stage, probability_cursor.phase,
-                            abort_flag, args.device_error, 52) ||
-              !ptx::mbarrier_wait_checked(full_bar + 8U * cursor.stage, cursor.phase, abort_flag,
-                            args.device_error, 53)) {
-            healthy = false;
-            break;
-          }
-          ptx::tcgen05_fence_after_thread_sync();
-          const uint32_t a_low = value_low + cursor.stage * (Shape::stage_bytes >> 4);
-          const uint32_t b_low =
-              probability_low + probability_cursor.stage * (Shape::probability_box_bytes >> 4);
+        const uint32_t a_low = value_low + cursor.stage * (Shape::stage_bytes >> 4);
+        const uint32_t b_low =
+            probability_low + probability_cursor.stage * (Shape::probability_box_bytes >> 4);
+        if (ptx::elect_one()) {
 #pragma unroll
           for (int slice = 0; slice < Shape::slices; ++slice)
             ptx::tcgen05_mma_f16_split(tmem_output + slice * padded_rows,
                                        a_low + slice * ((2 * Shape::value_box_bytes) >> 4),
                                        desc_high, b_low, desc_high, idesc, 0U);
-          accumulate = 1;
           ptx::tcgen05_commit(empty_bar + 8U * cursor.stage);
           ptx::tcgen05_commit(p_empty_bar + 8U * probability_cursor.stage);
-          cursor.advance();
-          probability_cursor.advance();
         }
-        const int key_groups = (item.rows_here + stream_value_keys - 1) / stream_value_keys;
-        for (int key_group = 0; key_group < key_groups; ++key_group) {
-          const int half = key_group & 1;
-          if (half == 0 &&
-              !ptx::mbarrier_wait_checked(p_full_bar + 8U * probability_cursor.stage, probability_cursor.phase,
-                            abort_flag, args.device_error, 52)) {
-            healthy = false;
-            break;
-          }
-          if (!ptx::mbarrier_wait_checked(full_bar + 8U * cursor.stage, cursor.phase, abort_flag,
-                            args.device_error, 53)) {
-            healthy = false;
-            break;
-          }
-          ptx::tcgen05_fence_after_thread_sync();
-          const uint32_t a_low = value_low + cursor.stage * (Shape::stage_bytes >> 4);
-          // 32 keys = 64 bytes along the 128-byte rows of the probability box.
-          const uint32_t b_low = probability_low +
-                                 probability_cursor.stage * (Shape::probability_box_bytes >> 4) +
-                                 half * 4;
+        __syncwarp();
+        accumulate = 1;
+        cursor.advance();
+        probability_cursor.advance();
+      }
+      const int key_groups = (item.rows_here + stream_value_keys - 1) / stream_value_keys;
+      for (int key_group = 0; key_group < key_groups; ++key_group) {
+        const int half = key_group & 1;
+        if (half == 0 &&
+            !wait(p_full_bar + 8U * probability_cursor.stage, probability_cursor.phase, 52))
+          break;
+        if (!wait(full_bar + 8U * cursor.stage, cursor.phase, 53))
+          break;
+        ptx::tcgen05_fence_after_thread_sync();
+        const uint32_t a_low = value_low + cursor.stage * (Shape::stage_bytes >> 4);
+        // 32 keys = 64 bytes along the 128-byte rows of the probability box.
+        const uint32_t b_low = probability_low +
+                               probability_cursor.stage * (Shape::probability_box_bytes >> 4) +
+                               half * 4;
+        const bool box_done = half == 1 || key_group + 1 == key_groups;
+        if (ptx::elect_one()) {
 #pragma unroll
           for (int step = 0; step < 2; ++step) {
 #pragma unroll
@@ -890,17 +892,19 @@ values_stream_kernel(const __grid_constant__ CUtensorMap value_map,
                   desc_high, b_low + 2 * step, desc_high, idesc, step > 0 ? 1U : accumulate);
             }
           }
-          accumulate = 1;
           ptx::tcgen05_commit(empty_bar + 8U * cursor.stage);
-          cursor.advance();
-          if (half == 1 || key_group + 1 == key_groups) {
+          if (box_done)
             ptx::tcgen05_commit(p_empty_bar + 8U * probability_cursor.stage);
-            probability_cursor.advance();
-          }
         }
-        if (healthy)
-          ptx::tcgen05_commit(o_full_bar + 8U * buffer);
+        __syncwarp();
+        accumulate = 1;
+        cursor.advance();
+        if (box_done)
+          probability_cursor.advance();
       }
+      if (healthy && ptx::elect_one())
+        ptx::tcgen05_commit(o_full_bar + 8U * buffer);
+      __syncwarp();
     }
   } else if (warp < 2 + values_output_warps) {
     // ---- output: O[component, row] -> fp32 chunk partials, or bf16 when there is one chunk.
