@@ -70,6 +70,11 @@ public:
     if (zero)
       require_cuda(cudaMemset(pointer_, 0, bytes_), "clear runner memory");
   }
+  void release() {
+    cudaFree(pointer_);
+    pointer_ = nullptr;
+    bytes_ = 0;
+  }
   template <typename T = void> T *get() const { return static_cast<T *>(pointer_); }
   size_t bytes() const { return bytes_; }
 
@@ -86,6 +91,10 @@ public:
   ~PinnedBuffer() { cudaFreeHost(pointer_); }
   void allocate(size_t bytes) {
     require_cuda(cudaMallocHost(&pointer_, bytes), "allocate pinned mailbox");
+  }
+  void release() {
+    cudaFreeHost(pointer_);
+    pointer_ = nullptr;
   }
   template <typename T> T *get() const { return static_cast<T *>(pointer_); }
 
@@ -1485,7 +1494,8 @@ PrefillSegment packed_segment(const Runner &runner, int slot, int first, int cou
   return segment;
 }
 
-void prepare_packed_prefill(Runner &runner) {
+// Row buffers of the packed steps (1.6 GB at the 31B widths and 24 slots), once a runner.
+void allocate_packed_prefill(Runner &runner) {
   const auto &config = runner.config;
   const size_t rows = packed_prefill_rows;
   const size_t row_hidden = rows * config.hidden_size * 2;
@@ -1527,7 +1537,14 @@ void prepare_packed_prefill(Runner &runner) {
     require_cuda(cudaMemcpy(runner.unit_scale.get(), &one, sizeof(float), cudaMemcpyHostToDevice),
                  "set unit scale");
   }
-  size_t partial_bytes = 0;
+  // The clears above run on the default stream, the steps on the runner's.
+  require_cuda(cudaStreamSynchronize(nullptr), "clear prefill buffers");
+}
+
+// The layers' weight maps, and the partial sums' buffer that their schedules need.
+void plan_packed_prefill(Runner &runner) {
+  const auto &config = runner.config;
+  size_t partial_bytes = 256;
   runner.q_layers.clear();
   for (size_t index = 0; index < runner.layers.size(); ++index) {
     const LayerState &layer = runner.layers[index];
@@ -1557,10 +1574,38 @@ void prepare_packed_prefill(Runner &runner) {
           runner.q_normed.get(),
           static_cast<const unsigned char *>(weights.qkv) +
               static_cast<size_t>(layer.query_width()) * config.hidden_size * 2,
-          packed_prefill_rows, config.hidden_size, last_key_value, 1, packed_prefill_rows);
+          packed_prefill_rows, config.hidden_size, layer.packed_width() - layer.query_width(), 1,
+          packed_prefill_rows);
     }
   }
-  runner.q_partials.allocate(std::max<size_t>(partial_bytes, 256));
+  // The schedules depend on the widths alone, so another set of weights needs no other buffer.
+  if (runner.q_partials.get() == nullptr)
+    runner.q_partials.allocate(partial_bytes);
+}
+
+// False, with the buffers given back, when the device has no room for them: the eight-token steps
+// then do the work.
+bool prepare_packed_prefill(Runner &runner) {
+  if (!packed_prefill_takes(runner))
+    return false;
+  try {
+    if (runner.q_hidden_a.get() == nullptr)
+      allocate_packed_prefill(runner);
+    plan_packed_prefill(runner);
+    return true;
+  } catch (const Failure &) {
+    for (DeviceBuffer *buffer :
+         {&runner.q_hidden_a, &runner.q_hidden_b, &runner.q_residual, &runner.q_normed,
+          &runner.q_pre_mlp, &runner.q_activated, &runner.q_packed, &runner.q_queries,
+          &runner.q_attention, &runner.q_projected, &runner.q_gate_up, &runner.q_partials,
+          &runner.q_staged, &runner.q_inputs, &runner.q_last_rows, &runner.q_last_normed,
+          &runner.q_last_hidden, &runner.q_key_value})
+      buffer->release();
+    runner.q_host_inputs.release();
+    runner.q_layers.clear();
+    cudaGetLastError();
+    return false;
+  }
 }
 
 // One BF16 forward over consecutive prompt rows of several slots, all of them made resident: the
@@ -2438,11 +2483,9 @@ extern "C" int carat_b200_runner_set_bf16_weights(carat_b200_runner *runner,
     }
     runner->bf16_layers.assign(layers, layers + layer_count);
     runner->prefill_plans.clear();
-    runner->packed_prefill = packed_prefill_takes(*runner);
-    if (runner->packed_prefill) {
-      prepare_packed_prefill(*runner);
+    runner->packed_prefill = prepare_packed_prefill(*runner);
+    if (runner->packed_prefill)
       return;
-    }
     if (runner->p_normed.get() == nullptr) {
       const size_t rows = maximum_rows;
       runner->p_normed.allocate(rows * runner->config.hidden_size * 2);
