@@ -11,6 +11,8 @@
 // memory and feeds to its tensor core; what is saved there holds weights in flight instead.
 // Above 256 rows (BF16 prefill) the same kernel is an ordinary tiled GEMM: the row tiles of a
 // feature tile are dealt to neighbouring pairs, so its weights come from HBM once and then from L2.
+// 2,048 bf16 rows: 5376 -> 43008 597 us (1.59 PFLOP/s), 21504 -> 5376 313 us with the fp32 pieces
+// (1.51), 5376 -> 16384 223 us (1.62); 256 rows of 5376 -> 43008 103 us, 119 on single CTAs.
 //
 // The kernel stands outside the chain of programmatic dependent launches: it neither starts before
 // the previous grid has ended nor lets the next one start before it has. Overlapped with large

@@ -16,7 +16,10 @@
 // fp32) takes half of tensor memory; for head_dim 512 two CTAs take 256 output components each and
 // both compute S (1.5 times the work of an undivided tile, which would need all of tensor memory).
 // The running maximum follows a row only when its scores outgrow it by a factor of 2^8, so O is
-// seldom rescaled; probabilities above one cost no precision in bf16.
+// seldom rescaled; probabilities above one cost no precision in bf16. 2,048 rows of an empty slot:
+// 95 us a sliding layer (32 query heads, 16 KV heads of 256), 307 us a global one (4 of 512); in
+// eight-token pieces past the first wrap a sliding layer took three launches of 4 to 10 us for
+// every eight rows.
 //
 // Key tiles begin at multiples of 128 positions whatever the step's rows are, a tile that a row
 // does not see leaves its state exactly as it was, and the decision to move the maximum is each
