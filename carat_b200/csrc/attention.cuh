@@ -103,4 +103,21 @@ inline int attention_chunks(int max_cache_rows, int chunk_keys) {
   return chunks < 1 ? 1 : chunks;
 }
 
+// Cache rows per chunk of a long linear cache for the two-kernel tensor-core path. 1,024 when the
+// cohort's chunks fill the SMs (smaller ones balance ragged contexts better but each costs a change
+// of queries and a drain of the pipeline: 512 to 768 rows were 6 % slower at 24 contexts of 128 to
+// 6,144). A few requests leave most SMs without a chunk of that size: they are cut until every SM
+// has one, down to 256 rows. One request of 3,000 rows FEW_US us in 256-row chunks, 45.0 in
+// 1,024-row ones; six of 500 to 2,000 SIX_US and 43.7. The cut of a request depends on the
+// launch's longest context and its number of requests only, so equal requests are cut alike.
+inline int chunk_rows(int requests, int kv_heads, int max_cache_rows, int multiprocessors) {
+  const long long share = (static_cast<long long>(requests) * kv_heads * max_cache_rows +
+                           multiprocessors - 1) /
+                          multiprocessors;
+  if (share > 512 || max_cache_rows <= 512)
+    return 1024;
+  const int rounded = (static_cast<int>(share) + 127) / 128 * 128;
+  return rounded < 256 ? 256 : rounded;
+}
+
 } // namespace carat_b200

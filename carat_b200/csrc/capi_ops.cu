@@ -286,7 +286,8 @@ int run_verify_attention(bool tensor_cores, const void *bf16_queries, const void
         check_cuda(cudaMalloc(&request_chunks, sizeof(int) * 1024), "allocate chunk counts") != 0)
       return -100;
     a.request_chunks = request_chunks;
-    constexpr int long_chunk_keys = 1024;
+    const int long_chunk_keys =
+        chunk_rows(requests, kv_heads, a.max_cache_rows, device_multiprocessors());
     if (!staged && a.max_cache_rows > long_chunk_keys) {
       // Long linear caches are cut into chunks like the runner does; the chunk partials live in
       // library scratch and are summed into the caller's output.

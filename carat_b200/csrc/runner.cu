@@ -777,6 +777,28 @@ const AttentionMaps *draft_attention_maps(Runner &runner, int assistant_layer) {
   return &runner.draft_maps.emplace(assistant_layer, maps).first->second;
 }
 
+// Chunks of a global layer's cache: smaller ones for a few requests on the tensor-core kernels
+// (attention->maps set), as far as the buffers for partial sums and statistics reach.
+void choose_chunks(const Runner &runner, AttentionArguments *attention, int query_width,
+                   size_t partial_bytes) {
+  attention->chunk_keys = global_chunk_keys;
+  attention->stats_stride = runner.stats_stride;
+  if (attention->maps != nullptr) {
+    const int rows_per_chunk =
+        chunk_rows(attention->requests, attention->kv_heads, attention->max_cache_rows,
+                   device_multiprocessors());
+    const size_t chunks =
+        static_cast<size_t>(attention_chunks(attention->max_cache_rows, rows_per_chunk));
+    const size_t row_chunks = chunks * attention->requests * attention->depth;
+    if (row_chunks * query_width * sizeof(float) <= partial_bytes &&
+        row_chunks * attention->query_heads * sizeof(float2) <= runner.attention_stats.bytes()) {
+      attention->chunk_keys = rows_per_chunk;
+      attention->stats_stride = static_cast<int>(chunks);
+    }
+  }
+  attention->chunks = attention_chunks(attention->max_cache_rows, attention->chunk_keys);
+}
+
 struct StepLayout {
   int *tokens;
   int *positions;
@@ -933,8 +955,6 @@ void verify_step(Runner &runner, const int *proposals, int requests, int depth,
       attention.window = 0;
       attention.max_cache_rows = longest + depth;
       attention.score_stride = runner.score_stride_global;
-      attention.chunk_keys = global_chunk_keys;
-      attention.chunks = attention_chunks(longest + depth, global_chunk_keys);
     } else {
       attention.window = config.sliding_window;
       // The rings change only in the commit at the end of the step.
@@ -952,6 +972,8 @@ void verify_step(Runner &runner, const int *proposals, int requests, int depth,
     attention.stats_stride = runner.stats_stride;
     attention.request_chunks = runner.request_chunks.get<int>();
     attention.maps = verify_attention_maps(runner, index, depth);
+    if (shape.global_attention)
+      choose_chunks(runner, &attention, layer.query_width(), runner.attention_partials.bytes());
     // The one-kernel attention leaves the largest |output| in the quantiser's (still zero) word.
     const bool amax_known = runner.attention_amax && attention.maps != nullptr &&
                             attention_tc_launches(attention) == 1;
