@@ -15,10 +15,15 @@
 // (1.51), 5376 -> 16384 223 us (1.62); 256 rows of 5376 -> 43008 103 us, 119 on single CTAs.
 //
 // The kernel stands outside the chain of programmatic dependent launches: it neither starts before
-// the previous grid has ended nor lets the next one start before it has. Overlapped with large
-// grids of small CTAs on both sides, launches of clusters stopped making progress now and then
-// (every few thousand launches; CTAs of a neighbour that wait for this grid can fill the SMs its
-// clusters still need). The overlap is worth one to two microseconds of a launch of 40 to 600.
+// the previous grid has ended nor lets the next one start before it has. Inside the chain, between
+// grids of thousands of small CTAs, launches stopped making progress once in a few thousand; why is
+// not known. (Launch order alone does not explain it: a dependent grid is admitted only when every
+// CTA of the one before it has started.) What reading found is an arrival that nothing waited for:
+// the commits that free the last ring stages arrive in the peer CTA too, and its only reason to stay
+// was the later commit of the accumulator. An arrival that comes after the peer has left lands in
+// the shared memory of whatever CTA runs there next, which inside the chain is already set up. Both
+// producers now wait for the last use of every stage before the pair parts. The overlap is worth
+// one to two microseconds of a launch of 40 to 600.
 //
 // Roles per CTA: warp 0 requests tiles by TMA (no multicast; both CTAs' copies complete on the
 // leader's barrier), warp 1 of the leader issues the MMAs, warps 2-5 of both finish their 128
@@ -187,7 +192,8 @@ pair_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
                  "r"(static_cast<uint32_t>(shape.tmem_columns))
                  : "memory");
     // No relinquish of the allocation permit: it would act for the pair, and could overtake the
-    // other CTA's allocation. The kernel has the SM's tensor memory to itself anyway.
+    // other CTA's allocation. Nothing waits for it: every other kernel here with tensor memory asks
+    // for more shared memory than this one leaves, so none is on the SM beside it.
   }
   ptx::tcgen05_fence_before_thread_sync();
   __syncthreads();
@@ -231,6 +237,22 @@ pair_linear_kernel(const __grid_constant__ CUtensorMap weight_map,
           if (++stage == stages) {
             stage = 0;
             phase ^= 1U;
+          }
+        }
+      }
+      if (healthy) {
+        // The commits that free a stage arrive in both CTAs, and this CTA may not leave before the
+        // last of them has: wait until each stage could be filled again.
+        uint32_t tail = stage;
+        uint32_t tail_phase = phase;
+        for (uint32_t turn = 0; turn < stages && healthy; ++turn) {
+          if (!ptx::mbarrier_wait_fast(empty_bar + 8U * tail, tail_phase ^ 1U)) {
+            healthy = false;
+            atomicExch(args.device_error, 1);
+          }
+          if (++tail == stages) {
+            tail = 0;
+            tail_phase ^= 1U;
           }
         }
       }

@@ -5,6 +5,8 @@ only), so a row's result may not depend on how many rows its call has: bit-equal
 Against fp32 the bar is the bf16 rounding of the output, 2^-9 relative to a value, plus the
 accumulation order; 4e-3 norm-wise is twice that rounding's worst case.
 """
+import ctypes
+
 import pytest
 import torch
 
@@ -55,3 +57,37 @@ def test_rows_do_not_depend_on_the_call_they_are_in(cuda_device, wide, rows, k, 
         want = ((x.view(torch.float8_e4m3fn).float() @ w.view(torch.float8_e4m3fn).float().t())
                 * (x_scale * w_scale))
     assert rms_relative_error(many, want) < 4e-3
+
+
+def test_kernels_that_follow_a_pair_on_its_sms(cuda_device):
+    """Pair launches of one and several tiles a pair, each followed at once by a kernel whose barriers
+    lie where the pair's lay: an arrival left over from the pair would count there. Every round leaves
+    the same bytes and no wait runs out."""
+    library = carat_b200.library()
+    generator = torch.Generator(device="cuda").manual_seed(3)
+    calls = []
+    for rows, k, n in ((256, 2048, 18944), (24, 1024, 5376), (200, 4096, 37888), (5, 512, 18944)):
+        x = torch.randn(rows, k, device="cuda", generator=generator).to(torch.bfloat16)
+        w = (torch.randn(n, k, device="cuda", generator=generator) * 0.02).to(torch.bfloat16)
+        out = torch.empty(rows, n, dtype=torch.bfloat16, device="cuda")
+        size = library.carat_b200_bf16_linear_workspace_bytes(rows, k, n)
+        calls.append((x, w, out, rows, k, n, torch.empty(max(size, 16), dtype=torch.uint8,
+                                                         device="cuda"), size))
+
+    def round_of_calls():
+        for x, w, out, rows, k, n, workspace, size in calls:
+            check(library.carat_b200_bf16_linear(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows,
+                                                 k, n, workspace.data_ptr(), size, None))
+
+    round_of_calls()
+    torch.cuda.synchronize()
+    first = [call[2].clone() for call in calls]
+    for _ in range(10):
+        for _ in range(50):
+            round_of_calls()
+        torch.cuda.synchronize()
+        for call, want in zip(calls, first):
+            assert torch.equal(call[2].view(torch.int16), want.view(torch.int16))
+    code = ctypes.c_int(0)
+    check(library.carat_b200_device_error(ctypes.byref(code)))
+    assert code.value == 0
