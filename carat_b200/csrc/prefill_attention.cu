@@ -183,6 +183,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap query_map,
     const uint32_t value_low =
         static_cast<uint32_t>(ptx::umma_desc_mn_major_sw128(ring, box_bytes));
     const uint32_t query_low = static_cast<uint32_t>(ptx::umma_desc_k_major_sw128(query_tiles));
+    const int unseen = (first_tile + tiles) * prefill_key_tile - (last + 1);
     uint32_t stage = 0;
     uint32_t phase = 0;
     bool healthy = true;
@@ -238,6 +239,17 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap query_map,
       for (int box = 0; box < value_boxes; ++box) {
         if (!wait(full_bar + 8U * stage, phase, 65))
           break;
+        if (j + 1 == tiles && unseen > 0) {
+          // Rows behind the tile's last token are whatever the cache holds there: an earlier
+          // prompt's, or another head's or slot's where capacity is not whole tiles. Their
+          // probabilities are 0, but 0 times an infinity is not: the rows are cleared. (A row is
+          // 128 bytes of a box; the swizzle moves 16-byte pieces within it.)
+          const uint32_t first = ring + stage * box_bytes + (prefill_key_tile - unseen) * 128;
+          for (int piece = lane; piece < unseen * 8; piece += 32)
+            ptx::store_shared_zero16(first + piece * 16);
+          ptx::fence_proxy_async();
+          __syncwarp();
+        }
         if (ptx::elect_one()) {
           const uint32_t b_low = value_low + stage * (box_bytes >> 4);
 #pragma unroll

@@ -72,3 +72,31 @@ def test_long_steps_match_the_oracle(cuda_device):
             assert rms_relative_error(keys[slot], oracle.keys[index][slot]) < 2e-2
             assert rms_relative_error(values[slot], oracle.values[index][slot]) < 2e-2
             assert helpers.cosine(keys[slot], oracle.keys[index][slot]) > 0.999
+
+
+@pytest.mark.parametrize("context", [1024, 1000])
+def test_rows_behind_the_last_token_do_not_count(cuda_device, context):
+    """Cache rows that a prompt has not reached hold what was there before, and where the context is
+    not whole key tiles the last tile reaches into the next head's and slot's rows: none of it may
+    show, not even as 0 times an infinity."""
+    config = cs.ModelConfig(CONFIG.hidden, CONFIG.intermediate, CONFIG.vocab, CONFIG.window, context,
+                            CONFIG.eps, CONFIG.layers)
+    lengths = [1, 130, 700, context]
+    texts = prompts(config, lengths, seed=21)
+    wanted = None
+    for fill in (0.0, float("nan"), float("inf")):
+        _, device = build(config, len(texts) + 1)
+        for index, layer in enumerate(config.layers):
+            rows = torch.full((len(texts) + 1, layer.kv_heads, config.capacity(index),
+                               layer.head_dim), fill, dtype=torch.bfloat16)
+            device.write_cache(0, index, rows)
+            device.write_cache(1, index, rows)
+        slots = list(range(len(texts)))
+        tokens = device.prefill_slots_chunks(slots, texts, context)
+        got = [state(config, device, slot, length) for slot, length in zip(slots, lengths)]
+        if wanted is None:
+            wanted = tokens, got
+            continue
+        assert tokens == wanted[0]
+        for have, want in zip(got, wanted[1]):
+            assert all(torch.equal(a, b) for a, b in zip(have, want))
