@@ -103,21 +103,24 @@ inline int attention_chunks(int max_cache_rows, int chunk_keys) {
   return chunks < 1 ? 1 : chunks;
 }
 
-// Cache rows per chunk of a long linear cache for the two-kernel tensor-core path. 1,024 when the
-// cohort's chunks fill the SMs (smaller ones balance ragged contexts better but each costs a change
-// of queries and a drain of the pipeline: 512 to 768 rows were 6 % slower at 24 contexts of 128 to
-// 6,144). A few requests leave most SMs without a chunk of that size: they are cut until every SM
-// has one, down to 256 rows. One request of 3,000 rows FEW_US us in 256-row chunks, 45.0 in
-// 1,024-row ones; six of 500 to 2,000 SIX_US and 43.7. The cut of a request depends on the
-// launch's longest context and its number of requests only, so equal requests are cut alike.
+// Cache rows per chunk of a long linear cache for the two-kernel tensor-core path. 1,024 where that
+// gives the SMs enough chunks: each costs a change of queries and a drain of the pipeline (24
+// contexts of 128 to 6,144: 512 to 768 rows are 6 % slower). A few requests leave most SMs without
+// a chunk of that size: they are cut into 256 to 512 rows when every chunk of the launch then still
+// has an SM to itself. Both kernels, cold L2, 32 / 4 heads of 512, five rows a request, us with the
+// rule and with 1,024 rows: one context of 1,000 42 and 58, of 3,000 44 and 58, of 8,000 50 and 58;
+// 500 to 2,000 six times 46 and 58. Where the rule stops: 900 twenty times (two chunks each would
+// not all find an SM) 60, 73 if cut; 5,000 four times (640 rows would fit) 62, 64 if cut.
+// The cut follows the launch's number of requests and its longest context, so equal requests of one
+// launch are cut alike; in launches of another size the fp32 sums of a request may be taken in
+// another order.
+constexpr int uncut_chunk_rows = 1024;
 inline int chunk_rows(int requests, int kv_heads, int max_cache_rows, int multiprocessors) {
-  const long long share = (static_cast<long long>(requests) * kv_heads * max_cache_rows +
-                           multiprocessors - 1) /
-                          multiprocessors;
-  if (share > 512 || max_cache_rows <= 512)
-    return 1024;
-  const int rounded = (static_cast<int>(share) + 127) / 128 * 128;
-  return rounded < 256 ? 256 : rounded;
+  const int chunks = multiprocessors / (requests * kv_heads);   // a request may have
+  if (chunks < 2)
+    return uncut_chunk_rows;
+  const int rows = ((max_cache_rows + chunks - 1) / chunks + 127) / 128 * 128;
+  return rows > 512 ? uncut_chunk_rows : rows < 256 ? 256 : rows;
 }
 
 } // namespace carat_b200

@@ -286,16 +286,31 @@ int run_verify_attention(bool tensor_cores, const void *bf16_queries, const void
         check_cuda(cudaMalloc(&request_chunks, sizeof(int) * 1024), "allocate chunk counts") != 0)
       return -100;
     a.request_chunks = request_chunks;
-    const int long_chunk_keys =
+    // Chunk partials: [chunks][rows][query_heads * head_dim] in library scratch.
+    const auto partials_need = [&](int chunk_keys) {
+      return sizeof(float) *
+             static_cast<size_t>(attention_chunks(a.max_cache_rows, chunk_keys)) * requests *
+             depth * query_heads * head_dim;
+    };
+    int long_chunk_keys =
         chunk_rows(requests, kv_heads, a.max_cache_rows, device_multiprocessors());
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (long_chunk_keys < uncut_chunk_rows &&
+        (partials_need(long_chunk_keys) > partial_bytes ||
+         score_rows * attention_chunks(a.max_cache_rows, long_chunk_keys) > stats_rows)) {
+      // A stream under capture cannot get more scratch: it keeps to the uncut form's.
+      if (cudaStreamIsCapturing(cuda_stream, &capturing) != cudaSuccess)
+        cudaGetLastError();
+      if (capturing != cudaStreamCaptureStatusNone)
+        long_chunk_keys = uncut_chunk_rows;
+    }
     if (!staged && a.max_cache_rows > long_chunk_keys) {
       // Long linear caches are cut into chunks like the runner does; the chunk partials live in
       // library scratch and are summed into the caller's output.
       a.chunk_keys = long_chunk_keys;
       a.chunks = attention_chunks(a.max_cache_rows, long_chunk_keys);
       a.sum_chunks = 1;
-      const size_t need = sizeof(float) * static_cast<size_t>(a.chunks) * requests * depth *
-                          query_heads * head_dim;
+      const size_t need = partials_need(long_chunk_keys);
       if (need > partial_bytes) {
         if (partials != nullptr)
           cudaFree(partials);

@@ -34,7 +34,7 @@ constexpr int prefill_pieces = 64;     // (slot, eight-token piece) entries one 
 // the tensor cores (0.9 us a row and 31B layer against 154 us to stream its weights).
 constexpr int packed_prefill_rows = 2048;
 constexpr int maximum_rows = 256;      // rows one FP8 linear launch accepts (24 slots x depth 9 = 216)
-constexpr int global_chunk_keys = 1024;
+constexpr int global_chunk_keys = uncut_chunk_rows;
 
 struct Failure {
   std::string message;

@@ -289,7 +289,10 @@ CARAT_B200_API int carat_b200_qkv_postprocess(const void *bf16_packed, const voi
  * of 8 and >= 16 + the participating cache rows rounded up to 128 (cache rows = min(max_position,
  * capacity) for a ring, max_position + depth for a linear cache).
  * head_dim 256 / 512 with capacity % 128 == 0 runs on tensor cores (tcgen05 + TMA), head_dim 64 on
- * CUDA cores. Replaces GemmCausalPrefillAttention::run_uniform_batch / run_uniform_ring_batch
+ * CUDA cores. On tensor cores a linear cache is summed in chunks whose size follows `requests`,
+ * kv_heads and max_position: equal requests of one call get equal results, a request's results in
+ * calls of another size may differ in the order of fp32 sums. Replaces
+ * GemmCausalPrefillAttention::run_uniform_batch / run_uniform_ring_batch
  * (include/carat/prefill_gemm_attention.h:24-47). */
 CARAT_B200_API int carat_b200_verify_attention(const void *bf16_queries, const void *bf16_key_caches,
                                 const void *bf16_value_caches, const void *bf16_new_keys,

@@ -1,0 +1,46 @@
+"""Rules by which launches are cut, checked on the host: compiled from the kernels' own headers."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SOURCE = """
+#include "attention.cuh"
+using namespace carat_b200;
+extern "C" int chunk(int requests, int kv_heads, int rows, int sms) {
+  return chunk_rows(requests, kv_heads, rows, sms);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    if shutil.which("g++") is None or shutil.which("nvcc") is None:
+        pytest.skip("no g++ or no CUDA headers")
+    cuda_home = os.environ.get("CUDA_HOME", os.path.dirname(os.path.dirname(shutil.which("nvcc"))))
+    folder = tmp_path_factory.mktemp("rules")
+    source, library = folder / "rules.cpp", folder / "rules.so"
+    source.write_text(SOURCE)
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-shared", "-fPIC", "-I",
+                    os.path.join(ROOT, "carat_b200", "csrc"), "-I",
+                    os.path.join(cuda_home, "include"), str(source), "-o", str(library)],
+                   check=True, timeout=120)
+    return ctypes.CDLL(str(library))
+
+
+@pytest.mark.parametrize("sms", [148, 132])
+def test_a_cut_context_leaves_every_chunk_an_sm(rules, sms):
+    for kv_heads in (1, 4, 16):
+        for requests in (1, 2, 5, 9, 18, 20, 24, 37, 1024):
+            for rows in (1, 255, 257, 513, 905, 1024, 1025, 3000, 5005, 8192, 30000, 262144):
+                chunk = rules.chunk(requests, kv_heads, rows, sms)
+                assert chunk % 128 == 0 and (256 <= chunk <= 512 or chunk == 1024)
+                if chunk != 1024:
+                    chunks = -(-rows // chunk)
+                    assert requests * kv_heads * chunks <= sms, (requests, kv_heads, rows)
+    assert rules.chunk(20, 4, 905, sms) == 1024      # two chunks a request: 160 on 148 SMs
+    assert rules.chunk(1, 4, 905, sms) == 256
