@@ -2,6 +2,7 @@
 
 #include "context.cuh"
 #include "launch.cuh"
+#include "row_parts.cuh"
 
 #include <cooperative_groups.h>
 #include <cstdint>
@@ -13,7 +14,6 @@ namespace cg = cooperative_groups;
 namespace carat_b200 {
 namespace {
 
-constexpr int row_threads = 512;
 constexpr int row_warps = row_threads / 32;
 
 enum class RowMode : int { embed_norm, norm, plain, post_attention, geglu, layer_output, embed_concat };
@@ -241,8 +241,9 @@ row_kernel(RowArguments a) {
   const size_t rows = gridDim.x / parts;
   const int width = a.width;
   const int part = static_cast<int>(blockIdx.x) - static_cast<int>(row) * parts;
-  const int column_base = part * (width / parts);
-  const int column_end = part + 1 == parts ? width : column_base + width / parts;
+  const int span = row_part_columns(width, parts);
+  const int column_base = part * span;
+  const int column_end = min(width, column_base + span);
   const float width_value = static_cast<float>(width);
   constexpr bool two_norms = mode == RowMode::post_attention || mode == RowMode::layer_output;
   constexpr bool one_norm = mode == RowMode::embed_norm || mode == RowMode::norm;
@@ -686,21 +687,11 @@ template <RowMode mode> int launch_rows(RowArguments arguments, int rows, cudaSt
     return -1;
   }
   int parts = 1;
-  if constexpr (mode == RowMode::geglu) {
-    // Wide rows: two CTAs a row when the halves stay multiples of eight columns and the grid
-    // still fits the device at once (checked by launch_rows_chunks).
-    if (bf16_only && rows > 148) {
-      // No grid to keep resident: parts of at most two column groups a thread, two CTAs a SM.
-      // 2,048 rows of 21,504: 107 us in one part, 86 in three.
-      while (arguments.width / parts > 2 * row_threads * 8 || arguments.width % (8 * parts) != 0)
-        ++parts;
-    } else if (arguments.width >= 8192 && arguments.width % 16 == 0 && rows <= 148) {
-      parts = 2;   // 2 * 148 CTAs of the two-per-SM variant fit
-    }
-  }
+  if constexpr (mode == RowMode::geglu)
+    parts = geglu_parts(rows, arguments.width, !bf16_only, device_multiprocessors());
   for (; parts >= 1; --parts) {
     arguments.parts = parts;
-    const int span = arguments.width / parts;
+    const int span = row_part_columns(arguments.width, parts);
     const int groups = (span / 8 + row_threads - 1) / row_threads;
     const int ctas = rows * parts;
     int status = -2;

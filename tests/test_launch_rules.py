@@ -10,7 +10,12 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 SOURCE = """
 #include "attention.cuh"
+#include "row_parts.cuh"
 using namespace carat_b200;
+extern "C" int part_columns(int width, int parts) { return row_part_columns(width, parts); }
+extern "C" int parts_of(int rows, int width, int resident, int sms) {
+  return geglu_parts(rows, width, resident != 0, sms);
+}
 extern "C" int chunk(int requests, int kv_heads, int rows, int sms) {
   return chunk_rows(requests, kv_heads, rows, sms);
 }
@@ -30,6 +35,22 @@ def rules(tmp_path_factory):
                     os.path.join(cuda_home, "include"), str(source), "-o", str(library)],
                    check=True, timeout=120)
     return ctypes.CDLL(str(library))
+
+
+@pytest.mark.parametrize("sms", [148, 132])
+@pytest.mark.parametrize("resident", [0, 1])
+def test_geglu_parts_cover_the_row_and_stay_few(rules, resident, sms):
+    # 8 x 1031 and 8 x 2687 have no divisor near the wanted part count.
+    for width in (8, 512, 8184, 8192, 8 * 1031, 16 * 1031, 21504, 8 * 2687, 43008, 65536 + 8):
+        for rows in (1, sms, sms + 1, 2048):
+            parts = rules.parts_of(rows, width, resident, sms)
+            assert 1 <= parts <= max(2, -(-width // 8192)), (width, rows)
+            span = rules.part_columns(width, parts)
+            assert span % 8 == 0 and (parts - 1) * span < width <= parts * span, (width, rows)
+            if resident:
+                assert rows * parts <= 2 * sms or parts == 1
+            elif rows > sms:
+                assert span <= 8192
 
 
 @pytest.mark.parametrize("sms", [148, 132])

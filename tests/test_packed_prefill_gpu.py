@@ -100,3 +100,21 @@ def test_rows_behind_the_last_token_do_not_count(cuda_device, context):
         assert tokens == wanted[0]
         for have, want in zip(got, wanted[1]):
             assert all(torch.equal(a, b) for a, b in zip(have, want))
+
+
+def test_a_feed_forward_width_without_small_divisors(cuda_device):
+    """16 x 1,031 columns: the GeGLU row kernel of a step of many rows takes unequal parts."""
+    config = cs.ModelConfig(256, 16 * 1031, 2048, 256, 512, 1e-6,
+                            [cs.LayerConfig("sliding", 4, 2, 256, 1e4, False),
+                             cs.LayerConfig("global", 8, 1, 512, 1e6, True)])
+    text = prompts(config, [400], seed=31)[0]
+    oracle, device = build(config, 2)
+    first = device.prefill_slot(0, text, chunk_tokens=512)        # 400 rows: three parts
+    assert device.prefill_slot(1, text, chunk_tokens=100) == first    # two
+    for have, want in zip(state(config, device, 1, 400), state(config, device, 0, 400)):
+        assert torch.equal(have, want)
+    oracle.prefill_slot_fp8(0, text, chunk=8)
+    for index in range(len(config.layers)):
+        capacity = config.capacity(index)
+        assert rms_relative_error(device.value_cache(index, capacity)[0],
+                                  oracle.values[index][0]) < 2e-2
