@@ -45,6 +45,14 @@ void require_cuda(cudaError_t result, const char *operation) {
     throw Failure{std::string(operation) + ": " + cudaGetErrorString(result)};
 }
 
+struct OutOfMemory : Failure {};
+
+void require_memory(cudaError_t result, const char *operation) {
+  if (result == cudaErrorMemoryAllocation)
+    throw OutOfMemory{{std::string(operation) + ": " + cudaGetErrorString(result)}};
+  require_cuda(result, operation);
+}
+
 void require_launch(int status, const char *operation) {
   if (status != 0) {
     const cudaError_t last = cudaGetLastError();
@@ -65,8 +73,9 @@ public:
   }
   ~DeviceBuffer() { cudaFree(pointer_); }
   void allocate(size_t bytes, bool zero = false) {
+    release();
     bytes_ = bytes < 256 ? 256 : bytes;
-    require_cuda(cudaMalloc(&pointer_, bytes_), "allocate runner memory");
+    require_memory(cudaMalloc(&pointer_, bytes_), "allocate runner memory");
     if (zero)
       require_cuda(cudaMemset(pointer_, 0, bytes_), "clear runner memory");
   }
@@ -90,7 +99,8 @@ public:
   PinnedBuffer &operator=(const PinnedBuffer &) = delete;
   ~PinnedBuffer() { cudaFreeHost(pointer_); }
   void allocate(size_t bytes) {
-    require_cuda(cudaMallocHost(&pointer_, bytes), "allocate pinned mailbox");
+    release();
+    require_memory(cudaMallocHost(&pointer_, bytes), "allocate pinned mailbox");
   }
   void release() {
     cudaFreeHost(pointer_);
@@ -1492,7 +1502,11 @@ int packed_prefill_tiles(const Runner &runner) {
   return std::min(most, 8 * (packed_prefill_rows + runner.batch)) + runner.batch;
 }
 
+// Attention shapes of the packed kernel, and whole rounds of tiles that CTA pairs can share (see
+// schedule_pairs).
 bool packed_prefill_takes(const Runner &runner) {
+  if (device_multiprocessors() % 2 != 0)
+    return false;
   for (const LayerState &layer : runner.layers) {
     if (!prefill_attention_takes(layer.shape.query_heads, layer.shape.kv_heads,
                                  layer.shape.head_dim))
@@ -1516,7 +1530,8 @@ PrefillSegment packed_segment(const Runner &runner, int slot, int first, int cou
   return segment;
 }
 
-// Row buffers of the packed steps (1.6 GB at the 31B widths and 24 slots), once a runner.
+// Row buffers of the packed steps (1.3 GB at the 31B widths and 24 slots, 0.54 of it the staging
+// rows that grow with the slots), once a runner.
 void allocate_packed_prefill(Runner &runner) {
   const auto &config = runner.config;
   const size_t rows = packed_prefill_rows;
@@ -1605,17 +1620,13 @@ void plan_packed_prefill(Runner &runner) {
     runner.q_partials.allocate(partial_bytes);
 }
 
-// False, with the buffers given back, when the device has no room for them: the eight-token steps
-// then do the work.
+// False for models that the packed steps do not take, and, with the buffers given back, when the
+// device has no room for them: the eight-token steps then do the work. Any other failure is the
+// caller's to know.
 bool prepare_packed_prefill(Runner &runner) {
   if (!packed_prefill_takes(runner))
     return false;
-  try {
-    if (runner.q_hidden_a.get() == nullptr)
-      allocate_packed_prefill(runner);
-    plan_packed_prefill(runner);
-    return true;
-  } catch (const Failure &) {
+  const auto give_back = [&runner] {
     for (DeviceBuffer *buffer :
          {&runner.q_hidden_a, &runner.q_hidden_b, &runner.q_residual, &runner.q_normed,
           &runner.q_pre_mlp, &runner.q_activated, &runner.q_packed, &runner.q_queries,
@@ -1626,7 +1637,18 @@ bool prepare_packed_prefill(Runner &runner) {
     runner.q_host_inputs.release();
     runner.q_layers.clear();
     cudaGetLastError();
+  };
+  try {
+    if (runner.q_hidden_a.get() == nullptr)
+      allocate_packed_prefill(runner);
+    plan_packed_prefill(runner);
+    return true;
+  } catch (const OutOfMemory &) {
+    give_back();
     return false;
+  } catch (...) {
+    give_back();
+    throw;
   }
 }
 
@@ -2503,19 +2525,23 @@ extern "C" int carat_b200_runner_set_bf16_weights(carat_b200_runner *runner,
         throw Failure{"invalid batch model runner shape"};
       }
     }
-    runner->bf16_layers.assign(layers, layers + layer_count);
     runner->prefill_plans.clear();
-    runner->packed_prefill = prepare_packed_prefill(*runner);
-    if (runner->packed_prefill)
-      return;
-    if (runner->p_normed.get() == nullptr) {
-      const size_t rows = maximum_rows;
-      runner->p_normed.allocate(rows * runner->config.hidden_size * 2);
-      runner->p_pre_mlp.allocate(rows * runner->config.hidden_size * 2);
-      runner->p_activated.allocate(rows * runner->config.intermediate_size * 2);
-      runner->p_step_inputs.allocate(sizeof(int) * (rows + 4 * prefill_pieces), true);
-      runner->p_host_inputs.allocate(sizeof(int) * (rows + 4 * prefill_pieces));
-      runner->p_request_chunks.allocate(sizeof(int) * prefill_pieces, true);
+    runner->packed_prefill = false;
+    try {
+      runner->bf16_layers.assign(layers, layers + layer_count);
+      runner->packed_prefill = prepare_packed_prefill(*runner);
+      if (!runner->packed_prefill && runner->p_request_chunks.get() == nullptr) {
+        const size_t rows = maximum_rows;
+        runner->p_normed.allocate(rows * runner->config.hidden_size * 2);
+        runner->p_pre_mlp.allocate(rows * runner->config.hidden_size * 2);
+        runner->p_activated.allocate(rows * runner->config.intermediate_size * 2);
+        runner->p_step_inputs.allocate(sizeof(int) * (rows + 4 * prefill_pieces), true);
+        runner->p_host_inputs.allocate(sizeof(int) * (rows + 4 * prefill_pieces));
+        runner->p_request_chunks.allocate(sizeof(int) * prefill_pieces, true);
+      }
+    } catch (...) {
+      runner->bf16_layers.clear();   // prefill without its buffers is refused
+      throw;
     }
   });
 }

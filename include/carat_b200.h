@@ -691,6 +691,12 @@ typedef struct carat_b200_layer_bf16_weights {
   const void *down;
 } carat_b200_layer_bf16_weights;
 
+/* The first call takes the row buffers of prefill steps of 2,048 rows from the device and keeps them
+ * for the runner's life: 1.3 GB at the 31B widths and 24 slots, of which 0.54 GB grow with slots x
+ * (window + 256). A host that plans its memory to the last GB leaves that much. Where they do not fit
+ * the call succeeds without them (and gives back what it had): prompts then walk eight tokens a request
+ * at a time, two to three times slower. Called again with room, it takes them. Any other failure is
+ * returned, and prefill refused until a call succeeds. */
 CARAT_B200_API int carat_b200_runner_set_bf16_weights(carat_b200_runner *runner,
                                                       const carat_b200_layer_bf16_weights *layers,
                                                       int layer_count);
@@ -705,9 +711,11 @@ CARAT_B200_API int carat_b200_runner_set_bf16_weights(carat_b200_runner *runner,
  * Replaces Gemma4BatchModelRunner::prefill_slots_chunks (and, with one slot, prefill_slot_chunk;
  * with chunk_tokens >= every remainder, prefill_slots_suffix's result for a cold cache):
  * include/carat/batch_model_runner.h:37-47, cuda/batch_model_runner.cu:1066-1125,1230-1355.
- * Inside, the chunks' rows are packed into forwards of up to 2,048 rows (models whose attention
- * shapes the packed path does not take, head_dim 64 for one, walk them eight tokens a request at a
- * time); rows of different requests never mix in bf16, so the cut does not change results. Needs
+ * Inside, the chunks' rows are packed into forwards of up to 2,048 rows; rows of different requests
+ * never mix in bf16 and every sum's order depends on a row's position alone, so the cut does not
+ * change results. Models whose attention shapes the packed path does not take (head_dim 64; query
+ * heads per KV head that do not divide 128) walk eight tokens a request at a time; there the cut does
+ * not change results up to the first ring wrap, and past it last bits only. Needs
  * carat_b200_runner_set_bf16_weights. */
 CARAT_B200_API int carat_b200_runner_prefill_slots_chunks(
     carat_b200_runner *runner, const int *slots, const int *const *token_ids,
