@@ -38,3 +38,25 @@ def test_rows_at_the_edges_of_the_variants(cuda_device, rows, k, n):
             * (x_scale * w_scale))
     assert rms_relative_error(got, want) < 4e-3
     assert torch.equal(got[:1].view(torch.int16), linear(1).view(torch.int16))
+
+
+@pytest.mark.parametrize("rows", [1, 96, 97, 160, 161, 224, 225])
+@pytest.mark.parametrize("k,n", [(2048, 5376), (1024, 20480), (520, 1000)])
+def test_bf16_rows_at_the_edges_of_the_variants(cuda_device, rows, k, n):
+    library = carat_b200.library()
+    generator = torch.Generator(device="cuda").manual_seed(k + n)
+    x = torch.randn(256, k, device="cuda", generator=generator).to(torch.bfloat16)
+    w = (torch.randn(n, k, device="cuda", generator=generator) * 0.02).to(torch.bfloat16)
+
+    def linear(count):
+        out = torch.full((count, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+        size = library.carat_b200_bf16_linear_workspace_bytes(count, k, n)
+        workspace = torch.empty(max(size, 16), dtype=torch.uint8, device="cuda")
+        check(library.carat_b200_bf16_linear(x.data_ptr(), w.data_ptr(), out.data_ptr(), count, k, n,
+                                             workspace.data_ptr(), size, None))
+        torch.cuda.synchronize()
+        return out
+
+    got = linear(rows)
+    assert rms_relative_error(got, x[:rows].float() @ w.float().t()) < 4e-3
+    assert torch.equal(got[:1].view(torch.int16), linear(1).view(torch.int16))

@@ -102,6 +102,31 @@ def test_rows_behind_the_last_token_do_not_count(cuda_device, context):
             assert all(torch.equal(a, b) for a, b in zip(have, want))
 
 
+def test_row_tiles_with_a_cut_tail_leave_the_same_bytes(cuda_device):
+    """gate_up of 152 feature tiles (a round of 148 SMs and a last one cut along K), o in K pieces:
+    together with the row tiles of more than 256 rows, every cut leaves the same bytes."""
+    config = cs.ModelConfig(512, 9728, 2048, 256, 1024, 1e-6,
+                            [cs.LayerConfig("sliding", 4, 2, 256, 1e4, False),
+                             cs.LayerConfig("global", 8, 1, 512, 1e6, True)])
+    length = 700
+    text, other = prompts(config, [length, 900], seed=29)
+    oracle, device = build(config, 5)
+    first = device.prefill_slot(0, text, chunk_tokens=1024)       # three row tiles
+    wanted = state(config, device, 0, length)
+    assert device.prefill_slot(1, text, chunk_tokens=300) == first
+    assert device.prefill_slot(2, text, chunk_tokens=67) == first
+    assert device.prefill_slots_chunks([4, 3], [other, text], 1024)[1] == first   # 1,600 rows
+    for slot in (1, 2, 3):
+        for have, want in zip(state(config, device, slot, length), wanted):
+            assert torch.equal(have, want), slot
+    oracle.prefill_slot_fp8(0, text, chunk=8)
+    for index in range(len(config.layers)):
+        capacity = config.capacity(index)
+        assert rms_relative_error(device.key_cache(index, capacity)[0], oracle.keys[index][0]) < 2e-2
+        assert rms_relative_error(device.value_cache(index, capacity)[0],
+                                  oracle.values[index][0]) < 2e-2
+
+
 def test_a_feed_forward_width_without_small_divisors(cuda_device):
     """16 x 1,031 columns: the GeGLU row kernel of a step of many rows takes unequal parts."""
     config = cs.ModelConfig(256, 16 * 1031, 2048, 256, 512, 1e-6,
