@@ -44,24 +44,28 @@ def test_prompts_match_the_oracle(cuda_device):
 @pytest.mark.parametrize("length", [9, 100, 256, 640])
 def test_cuts_of_a_prompt(cuda_device, length):
     """Up to the first wrap every cut leaves the same bytes. Past it a row's sums begin with the rows of
-    its own piece, so the pieces of another cut may differ in last bits."""
+    its own piece, and where pieces begin depends on the cut and on the prompts beside this one: fp32
+    sums in another order, rounded to bf16, through three layers (the bars of the comparison with the
+    oracle)."""
     text = prompts(CONFIG, [length], seed=length)[0]
     other = prompts(CONFIG, [300], seed=5)[0]
     _, device = build(CONFIG, 3)
-    first = device.prefill_slot(0, text, chunk_tokens=1024)
+    tokens = [device.prefill_slot(0, text, chunk_tokens=1024)]
     wanted = state(CONFIG, device, 0, length)
-    second = device.prefill_slot(1, text, chunk_tokens=37)
+    tokens.append(device.prefill_slot(1, text, chunk_tokens=37))
     device.reset_slot(0)
-    assert device.prefill_slots_chunks([2, 0], [text, other], 1000)[0] == first   # same pieces
-    for have, want in zip(state(CONFIG, device, 2, length), wanted):
-        assert torch.equal(have, want), length
-    if length <= CONFIG.window:
-        assert second == first
-    for have, want in zip(state(CONFIG, device, 1, length), wanted):
-        if length <= CONFIG.window:
-            assert torch.equal(have, want), length
-        else:
-            assert rms_relative_error(have.view(torch.bfloat16), want.view(torch.bfloat16)) < 4e-2
+    tokens.append(device.prefill_slots_chunks([2, 0], [text, other], 1000)[0])
+    whole = length <= CONFIG.window
+    assert not whole or len(set(tokens)) == 1
+    for slot in (1, 2):
+        *caches, hidden = zip(state(CONFIG, device, slot, length), wanted)
+        for have, want in caches:
+            if whole:
+                assert torch.equal(have, want), (length, slot)
+            assert rms_relative_error(have.view(torch.bfloat16), want.view(torch.bfloat16)) < 2e-2
+        if whole:
+            assert torch.equal(*hidden)
+        assert cosine(hidden[0].view(torch.bfloat16), hidden[1].view(torch.bfloat16)) > 0.999
 
 
 def test_a_device_without_room_for_the_packed_buffers(cuda_device):
