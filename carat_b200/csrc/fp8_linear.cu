@@ -665,8 +665,7 @@ finalize_vector_kernel(const float *partial, const float *input_scale, const flo
 // calls too small to give the other kernel a few blocks a SM (with the linear: 24 rows of 5376 in
 // three pieces 11.3 us against 12.1, 72 rows 12.9 against 13.4, 120 rows of 1024 in eighteen 10.3
 // against 12.0).
-// `whole`: the pieces cover whole output rows, so an index needs no division, which is a good part of
-// a small call.
+// `whole`: the pieces cover whole output rows, so an index needs no division.
 template <bool whole>
 __global__ void finalize_column_kernel(const float *partial, const float *input_scale,
                                        const float *weight_scale, __nv_bfloat16 *output,
@@ -762,10 +761,10 @@ int launch_variant(const LinearPlan &plan, const KernelArguments &arguments, cud
              : -11;
 }
 
-// Rows in steps of 32: what a call loads, multiplies and holds in its ring is close to its rows.
-// With steps of 64 beyond 64, 216 rows (24 slots, nine proposals) filled 256 and left room for four
-// stages instead of five: e4m3 21504 -> 5376 35.5 us instead of 29.6, 5376 -> 43008 64.3 instead of
-// 49.6; 150 rows 50.8 instead of 46.9, 72 rows 41.8 instead of 40.3.
+// Rows in steps of 32: what a call loads, multiplies and holds in its ring is close to its rows. The
+// step to the next variant costs, e4m3 21504 -> 5376 back to back: 64 to 65 rows 23.8 to 24.6 us, 96 to
+// 97 25.1 to 25.7, 160 to 161 26.7 to 27.4, 224 to 225 29.0 to 31.4 (a ring of four stages instead of
+// five); with steps of 64 beyond 64 rows all calls would pay for the next multiple of 64.
 template <int mode, bool wide>
 int launch_rows_bucket(const LinearPlan &plan, const KernelArguments &arguments,
                        cudaStream_t stream) {
@@ -812,12 +811,16 @@ int launch_planned(const LinearPlan &plan, const KernelArguments &arguments, cud
 
 // Single CTAs or pairs. More rows than a tile holds need the pairs' row tiles. Up to 256 rows the
 // pairs pay where the activation half of a tile is what an SM has too much of, K is not cut (their
-// start and end cost two cluster barriers) and a tile is long enough to hide those: bf16
-// 5376 -> 43008 at 256 rows 103 us against 119, 192 rows 85 against 91, 128 rows 79 against 79,
-// 24 rows 70 against 68; e4m3 256 rows 59 to 64 against 67 to 73, 192 rows 54 against 54; but
-// bf16 1024 -> 262144 (16 blocks of K) 240 against 235 at 256 rows. A launch long enough to forget
-// its start (the LM head: eight rounds of tiles and more) has them from 97 rows on: e4m3
-// 5376 -> 262144 120 rows 225 against 236, 160 rows 242 against 256, but 72 rows 216 against 216.
+// start and end cost two cluster barriers) and a tile is long enough to hide those. The line lies at
+// 160 rows. Pairs and single CTAs in us: e4m3 5376 -> 43008 back to back 256 rows 55.0 and 63.2, 216
+// rows 51.1 and 56.5, 192 rows 48.8 and 52.9, 161 rows 47.2 and 50.3; bf16, cold, 256 rows 99 and 116,
+// 192 rows 91 and 97, 161 rows 89 and 97. A call of its own would have them from about 110 rows on (128
+// rows 44.3 and 45.4, 97 rows 45.4 and 45.0), but in a chain of dependent launches they give up the overlap
+// with both neighbours: verify steps of six layers take 1,462 and 1,461 us at 135 rows, 1,614 and 1,633
+// at 153, 1,665 and 1,747 at 162, 1,708 and 1,748 at 180. Few blocks of K: bf16 1024 -> 262144 (16)
+// 240 and 235 at 256 rows. A launch long enough to forget its start (the LM head: eight rounds of tiles
+// and more) has them from 97 rows on: e4m3 5376 -> 262144 back to back 97 rows 217 and 222, 120 rows
+// 219 and 227, 160 rows 243 and 248, 192 rows 272 and 282; but 72 rows 216 and 216.
 bool schedule_plain(LinearPlan *plan, int rows, int input_width, int output_width,
                     int requested_splits, int element_bytes) {
   schedule_linear(plan, rows, input_width, output_width, requested_splits, element_bytes);
@@ -825,7 +828,7 @@ bool schedule_plain(LinearPlan *plan, int rows, int input_width, int output_widt
   if (rows > 256)
     return schedule_pairs(plan);
   if (plan->splits == 1 && plan->tiles >= plan->ctas / 2 && plan->k_blocks >= 32 &&
-      (rows > (element_bytes == 2 ? 160 : 192) || (rows > 96 && plan->tiles >= 8 * plan->ctas))) {
+      (rows > 160 || (rows > 96 && plan->tiles >= 8 * plan->ctas))) {
     schedule_pairs(plan);   // keeps the plan when it cannot
   }
   return true;
@@ -1014,7 +1017,8 @@ int launch_linear_finalize(const float *partial, const float *input_scale,
                            int width, int output_width, int first_column, cudaStream_t stream) {
   auto *output = static_cast<__nv_bfloat16 *>(bf16_output);
   const size_t elements = static_cast<size_t>(rows) * width;
-  const bool vectors = elements > 512 * 1024 && width % 8 == 0 && output_width % 8 == 0 && first_column % 8 == 0 &&
+  const bool vectors = elements > 512 * 1024 && width % 8 == 0 && output_width % 8 == 0 &&
+                       first_column % 8 == 0 &&
                        reinterpret_cast<uintptr_t>(partial) % 16 == 0 &&
                        reinterpret_cast<uintptr_t>(output) % 16 == 0 && elements / 8 < 0x7FFFFF00U;
   if (vectors) {

@@ -17,8 +17,7 @@ from helpers import rms_relative_error
 pytestmark = pytest.mark.gpu
 
 # (rows of the wide call, K, N): edges of the row tile, odd 128-feature tile counts, a K-cut tail,
-# a last feature tile that is half empty, K that is not a whole number of blocks. (161 rows take pairs
-# in bf16 only, from 193 on both types do.)
+# a last feature tile that is half empty, K that is not a whole number of blocks.
 SHAPES = [(161, 4096, 16384), (193, 4096, 16384), (193, 5376, 43008), (224, 4112, 19200), (256, 5376, 18944 + 128),
           (255, 8192, 9472 + 64)]
 
