@@ -879,7 +879,9 @@ int make_linear_plan(LinearPlan *plan, const void *fp8_input, const void *fp8_we
   if (element_bytes != 1 && element_bytes != 2)
     return fail("invalid FP8 linear shape", -1);
   if (rows > most_rows)
-    return fail("FP8 linear supports at most 256 rows", -2);
+    return fail(most_rows <= 256 ? "FP8 linear supports at most 256 rows"
+                                 : "more rows than a step of this linear takes",
+                -2);
   if (input_width * element_bytes % 16 != 0)
     return fail("FP8 linear input width must be a multiple of 16", -3);
   if ((reinterpret_cast<uintptr_t>(fp8_input) & 15U) != 0 ||

@@ -7,16 +7,17 @@
 // Same swapped-operand weight stream as the e4m3 linear (128 output features = UMMA M, padded
 // activation rows = UMMA N, persistent CTAs walking tile x K-piece items), with one more stage
 // between TMA and the tensor core: the 4-bit codes cannot feed tcgen05.mma together with bf16
-// activations, so two or three groups of four warps turn every [128 features x 128 K] tile of codes (8 KB, plus its 128
-// group scales) into bf16 and store it into tensor memory (tcgen05.st), where the MMA warp takes
-// it as the A operand (kind::f16, A in TMEM) against the bf16 activation boxes in shared memory.
+// activations, so two or three groups of four warps turn every [128 features x 128 K] tile of codes
+// (8 KB, plus its 128 group scales) into bf16 and store it into tensor memory (tcgen05.st), where the
+// MMA warp takes it as the A operand (kind::f16, A in TMEM) against the bf16 activation boxes in
+// shared memory.
 // Keeping the converted weights out of shared memory matters: written there and read back by the
 // tensor core they cost 64 KB of shared-memory traffic per K block on top of the 72 KB of TMA
 // writes and B-operand reads, and the kernel was bound by shared-memory bandwidth (measured: no
 // change when either TMA stream was switched off). Rings: codes + scales (TMA, deep, small),
 // activations (TMA from L2), converted weights (four TMEM buffers of 64 columns, filled by two or
-// three groups of four warps on consecutive K blocks). The codes are read from HBM exactly once; that is
-// half the bytes of the e4m3 weights, but the kernel is bound on the SM: at 128 padded rows the
+// three groups of four warps on consecutive K blocks). The codes are read from HBM exactly once; that
+// is half the bytes of the e4m3 weights, but the kernel is bound on the SM: at 128 padded rows the
 // eight bf16 MMAs of a K block keep the tensor pipe busy about 700 cycles (an e4m3 MMA consumes 32
 // bytes of a weight row, a bf16 MMA over 4-bit codes 8), and below 64 rows the conversion (shift,
 // mask-or, bf16 subtract, bf16 multiply per pair of codes) is the limit.
@@ -521,8 +522,8 @@ int launch_variant(const Int4LinearPlan &plan, const KernelArguments &arguments,
                     arguments.tail_tiles * arguments.tail_splits;
   const int ctas = items < schedule.ctas ? items : schedule.ctas;
   return launch_chained(int4_linear_kernel<padded_rows, mode>, dim3(static_cast<unsigned>(ctas)),
-                        dim3(Layout<padded_rows>::threads), dynamic_bytes, stream, false, schedule.weight_map,
-                        plan.scale_map, schedule.input_map, arguments,
+                        dim3(Layout<padded_rows>::threads), dynamic_bytes, stream, false,
+                        schedule.weight_map, plan.scale_map, schedule.input_map, arguments,
                         plan.group_shift) == cudaSuccess
              ? 0
              : -11;
@@ -681,8 +682,9 @@ int launch_int4_linear_bf16(const Int4LinearPlan &plan, void *bf16_output, float
     if (status != 0)
       return status;
     const int tail_width = schedule.tail_tiles * tile_features;
-    return launch_linear_finalize(partial, nullptr, nullptr, bf16_output, schedule.tail_splits, schedule.rows, tail_width,
-                           schedule.output_width, schedule.output_width - tail_width, stream);
+    return launch_linear_finalize(partial, nullptr, nullptr, bf16_output, schedule.tail_splits,
+                                  schedule.rows, tail_width, schedule.output_width,
+                                  schedule.output_width - tail_width, stream);
   }
   if (schedule.splits == 1) {
     KernelArguments arguments = base_arguments(schedule, device_error, false);
@@ -692,8 +694,9 @@ int launch_int4_linear_bf16(const Int4LinearPlan &plan, void *bf16_output, float
   const int status = launch_int4_linear_partial(plan, partial, device_error, stream);
   if (status != 0)
     return status;
-  return launch_linear_finalize(partial, nullptr, nullptr, bf16_output, schedule.splits, schedule.rows,
-                         schedule.output_width, schedule.output_width, 0, stream);
+  return launch_linear_finalize(partial, nullptr, nullptr, bf16_output, schedule.splits,
+                                schedule.rows, schedule.output_width, schedule.output_width, 0,
+                                stream);
 }
 
 int launch_int4_linear_simt_check(const void *bf16_input, const void *packed_row_major,

@@ -10,8 +10,8 @@ namespace carat_b200 {
 
 constexpr int pair_features = 256;   // UMMA M of a CTA pair: output features per tile
 
-// Activation rows of one tile (UMMA N, a multiple of 16, with e4m3 operands of 32) for a call of `rows` rows: one tile up to
-// 256 rows, above that equal tiles of at most 256.
+// Activation rows of one tile (UMMA N, a multiple of 16, with e4m3 operands of 32) for a call of
+// `rows` rows: one tile up to 256 rows, above that equal tiles of at most 256.
 inline int pair_row_tiles(int rows) { return (rows + 255) / 256; }
 inline int pair_tile_rows(int rows, int element_bytes) {
   const int granule = element_bytes == 2 ? 16 : 32;

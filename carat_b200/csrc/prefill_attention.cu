@@ -16,7 +16,8 @@
 // fp32) takes half of tensor memory; for head_dim 512 two CTAs take 256 output components each and
 // both compute S (1.5 times the work of an undivided tile, which would need all of tensor memory).
 // The running maximum follows a row only when its scores outgrow it by a factor of 2^8, so O is
-// seldom rescaled; probabilities above one cost no precision in bf16. 2,048 rows of an empty slot:
+// seldom rescaled (lazy rescaling, a published method of recent FlashAttention kernels);
+// probabilities above one cost no precision in bf16. 2,048 rows of an empty slot:
 // 95 us a sliding layer (32 query heads, 16 KV heads of 256), 307 us a global one (4 of 512); in
 // eight-token pieces past the first wrap a sliding layer took three launches of 4 to 10 us for
 // every eight rows.
@@ -560,7 +561,10 @@ int launch_prefill_gather(const PrefillGatherArguments &a, cudaStream_t stream) 
       a.head_stride % 8 != 0) {
     return -1;
   }
-  const dim3 grid(a.segment_count == 1 ? 296 : 74, static_cast<unsigned>(a.segment_count));
+  // Two blocks a SM for a lone segment, half a block a SM and segment for several.
+  const int multiprocessors = device_multiprocessors();
+  const dim3 grid(a.segment_count == 1 ? 2 * multiprocessors : (multiprocessors + 1) / 2,
+                  static_cast<unsigned>(a.segment_count));
   return launch_chained(prefill_gather_kernel, grid, dim3(256), 0, stream, false, a) == cudaSuccess
              ? 0
              : -11;
