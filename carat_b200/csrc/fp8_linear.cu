@@ -665,6 +665,8 @@ finalize_vector_kernel(const float *partial, const float *input_scale, const flo
 // calls too small to give the other kernel a few blocks a SM (with the linear: 24 rows of 5376 in
 // three pieces 11.3 us against 12.1, 72 rows 12.9 against 13.4, 120 rows of 1024 in eighteen 10.3
 // against 12.0).
+// `whole`: the pieces cover whole output rows, so an index needs no division.
+template <bool whole>
 __global__ void finalize_column_kernel(const float *partial, const float *input_scale,
                                        const float *weight_scale, __nv_bfloat16 *output,
                                        int pieces, int rows, int width, int output_width,
@@ -689,7 +691,7 @@ __global__ void finalize_column_kernel(const float *partial, const float *input_
           sum += piece[offset];
     }
     size_t destination = index;
-    if (width != output_width) {   // a division is a good part of a small call
+    if constexpr (!whole) {
       const size_t row = index / width;
       destination = row * output_width + first_column + (index - row * width);
     }
@@ -1031,7 +1033,9 @@ int launch_linear_finalize(const float *partial, const float *input_scale,
   }
   const size_t wanted = (elements + 255) / 256;
   const unsigned blocks = static_cast<unsigned>(wanted < 1184 ? wanted : 1184);
-  return launch_chained(finalize_column_kernel, dim3(blocks), dim3(256), 0, stream, false, partial,
+  return launch_chained(width == output_width ? finalize_column_kernel<true>
+                                              : finalize_column_kernel<false>,
+                        dim3(blocks), dim3(256), 0, stream, false, partial,
                         input_scale, weight_scale, output, pieces, rows, width, output_width,
                         first_column) == cudaSuccess
              ? 0
