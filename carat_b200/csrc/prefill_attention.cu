@@ -62,7 +62,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float low, float high) {
   return *reinterpret_cast<const uint32_t *>(&pair);
 }
 
-template <int head_dim>
+// `clears`: the key matrix is a cache, whose rows behind a tile's last token are whatever an earlier
+// prompt left there, or another head's or slot's where capacity is not whole tiles. Their
+// probabilities are 0, but 0 times an infinity is not: the MMA warp clears them in shared memory, in
+// the last key tile of each query tile. (The staging buffer of the sliding layers is clear there.)
+template <int head_dim, bool clears>
 __global__ void __launch_bounds__(prefill_threads, 1)
 prefill_attention_kernel(const __grid_constant__ CUtensorMap query_map,
                          const __grid_constant__ CUtensorMap key_map,
@@ -184,7 +188,6 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap query_map,
     const uint32_t value_low =
         static_cast<uint32_t>(ptx::umma_desc_mn_major_sw128(ring, box_bytes));
     const uint32_t query_low = static_cast<uint32_t>(ptx::umma_desc_k_major_sw128(query_tiles));
-    const int unseen = (first_tile + tiles) * prefill_key_tile - (last + 1);
     uint32_t stage = 0;
     uint32_t phase = 0;
     bool healthy = true;
@@ -240,16 +243,21 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap query_map,
       for (int box = 0; box < value_boxes; ++box) {
         if (!wait(full_bar + 8U * stage, phase, 65))
           break;
-        if (j + 1 == tiles && unseen > 0) {
-          // Rows behind the tile's last token are whatever the cache holds there: an earlier
-          // prompt's, or another head's or slot's where capacity is not whole tiles. Their
-          // probabilities are 0, but 0 times an infinity is not: the rows are cleared. (A row is
-          // 128 bytes of a box; the swizzle moves 16-byte pieces within it.)
-          const uint32_t first = ring + stage * box_bytes + (prefill_key_tile - unseen) * 128;
-          for (int piece = lane; piece < unseen * 8; piece += 32)
-            ptx::store_shared_zero16(first + piece * 16);
-          ptx::fence_proxy_async();
-          __syncwarp();
+        if constexpr (clears) {
+          if (j + 1 == tiles) {
+            // A row is 128 bytes of a box (the swizzle moves 16-byte pieces within it), four rows a
+            // turn of the warp, from the box's end.
+            const int unseen = (first_tile + tiles) * prefill_key_tile - (last + 1);
+            const uint32_t end = ring + (stage + 1) * box_bytes;
+            uint32_t address = end - 512 + lane * 16;
+            const uint32_t least = end - unseen * 128;
+#pragma unroll 8
+            for (int turn = 0; turn < prefill_key_tile / 4; ++turn, address -= 512)
+              if (address >= least)
+                ptx::store_shared_zero16(address);
+            ptx::fence_proxy_async();
+            __syncwarp();
+          }
         }
         if (ptx::elect_one()) {
           const uint32_t b_low = value_low + stage * (box_bytes >> 4);
@@ -491,21 +499,21 @@ bool encode_rows(CUtensorMap *map, const void *base, long long rows, int columns
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int head_dim>
-int launch_head_dim(const PrefillAttentionMaps &maps, const PrefillAttentionArguments &a,
-                    cudaStream_t stream) {
+template <int head_dim, bool clears>
+int launch_variant(const PrefillAttentionMaps &maps, const PrefillAttentionArguments &a,
+                   cudaStream_t stream) {
   constexpr int dynamic_bytes = (head_dim / 64 + ring_boxes(head_dim)) * box_bytes + 1024;
   static PerDeviceOnce configured;
   if (configured.run([] {
-        return cudaFuncSetAttribute(prefill_attention_kernel<head_dim>,
+        return cudaFuncSetAttribute(prefill_attention_kernel<head_dim, clears>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic_bytes);
       }) != cudaSuccess) {
     return -10;
   }
   const int blocks = a.tile_count * a.kv_heads * (head_dim / 256);
-  return launch_chained(prefill_attention_kernel<head_dim>, dim3(static_cast<unsigned>(blocks)),
-                        dim3(prefill_threads), dynamic_bytes, stream, false, maps.queries,
-                        maps.keys, maps.values, a) == cudaSuccess
+  return launch_chained(prefill_attention_kernel<head_dim, clears>,
+                        dim3(static_cast<unsigned>(blocks)), dim3(prefill_threads), dynamic_bytes,
+                        stream, false, maps.queries, maps.keys, maps.values, a) == cudaSuccess
              ? 0
              : -11;
 }
@@ -550,8 +558,12 @@ int launch_prefill_attention(const PrefillAttentionMaps &maps, const PrefillAtte
       !prefill_attention_takes(a.query_heads, a.kv_heads, a.head_dim)) {
     return -1;
   }
-  return a.head_dim == 256 ? launch_head_dim<256>(maps, a, stream)
-                           : launch_head_dim<512>(maps, a, stream);
+  if (a.window > 0) {
+    return a.head_dim == 256 ? launch_variant<256, false>(maps, a, stream)
+                             : launch_variant<512, false>(maps, a, stream);
+  }
+  return a.head_dim == 256 ? launch_variant<256, true>(maps, a, stream)
+                           : launch_variant<512, true>(maps, a, stream);
 }
 
 int launch_prefill_gather(const PrefillGatherArguments &a, cudaStream_t stream) {

@@ -236,7 +236,7 @@ row_kernel(RowArguments a) {
 
   // Modes without a row-wide reduction (GeGLU) may cut a row into `parts` column ranges, one CTA
   // each, so that a wide row does not sit in a single CTA.
-  const int parts = a.parts > 1 ? a.parts : 1;
+  const int parts = mode == RowMode::geglu && a.parts > 1 ? a.parts : 1;
   const size_t row = blockIdx.x / parts;
   const size_t rows = gridDim.x / parts;
   const int width = a.width;
