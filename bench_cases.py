@@ -178,9 +178,10 @@ def global_ragged(launches=3):
               contexts=bench.context_lengths(seed=3), launches=launches)
 
 
-def _period_model(slots, max_context, with_assistant):
+def _period_model(slots, max_context, with_assistant, extra_layers=0):
     """One period of the 31B layer pattern (five sliding layers and one global layer at the real
-    widths, vocabulary 262144) with bf16 and e4m3 weights, and the reference-shaped drafter."""
+    widths, vocabulary 262144; `extra_layers` more begin another period) with bf16 and e4m3 weights, and
+    the reference-shaped drafter."""
     import carat_b200
     generator = torch.Generator(device="cuda").manual_seed(0)
 
@@ -198,6 +199,7 @@ def _period_model(slots, max_context, with_assistant):
 
     layers = [carat_b200.Gemma4LayerConfig("sliding", 32, 16, 256, 1e4, False) for _ in range(5)]
     layers.append(carat_b200.Gemma4LayerConfig("global", 32, 4, 512, 1e6, True))
+    layers += layers[:extra_layers]
     config = carat_b200.Gemma4Config(5376, 21504, 262144, 1024, 1e-6, layers)
     hidden, inter = config.hidden_size, config.intermediate_size
     bf16 = {"token_embedding": matrix(config.vocabulary_size, hidden), "final_norm": ones(hidden)}
@@ -241,14 +243,20 @@ def _period_model(slots, max_context, with_assistant):
     return config, runner, weight_bytes, (weights, fp8, a_weights, a_fp8)
 
 
-def prefill(launches=6, slots=24, chunk=8, context=1024):
-    """BF16 prompt prefill on one period of the 31B layer pattern: `slots` prompts advance `chunk`
-    tokens a call from `context` resident tokens. Prints the device time per call, the same figure
-    for the 60-layer model (ten periods: extrapolated, the LM head is outside the timed calls) and
-    the share of the bf16 weight stream's roofline."""
+def prefill(launches=6, slots=24, chunk=64, context=1024):
+    """BF16 prompt prefill on one period of the 31B layer pattern and a seventh layer: `slots` prompts
+    advance `chunk` tokens a call, packed into one step (24 x 64 = 1,536 rows), from `context` resident
+    tokens, past the first ring wrap. A step makes only K and V of a model's last layer where no prompt
+    ends in it, so the seventh layer keeps the period whole. Prints the device time per call, the same
+    figure for the 60-layer model (ten periods: extrapolated) and the rate of the period's
+    projections."""
     # A multiple of 128 rows, like the server's 8192: the tensor-core attention needs that.
     max_context = (context + chunk * (launches + 2) + 64 + 127) // 128 * 128
-    config, runner, weight_bytes, keep = _period_model(slots, max_context, with_assistant=False)
+    config, runner, weight_bytes, keep = _period_model(slots, max_context, with_assistant=False,
+                                                       extra_layers=1)
+    last = config.layers[-1]
+    weight_bytes -= 2 * config.hidden_size * (last.packed_width() + last.query_width()
+                                              + 3 * config.intermediate_size)
     runner.seed_empty_cache_for_benchmark(context)
     tokens = torch.randint(3, config.vocabulary_size, (slots, max_context),
                            generator=torch.Generator().manual_seed(1)).tolist()
@@ -272,23 +280,25 @@ def prefill(launches=6, slots=24, chunk=8, context=1024):
         wall = start.elapsed_time(stop) / (launches - 1)
         period = device_ms / (launches - 1)
         rows = slots * chunk
-        roofline = weight_bytes / 1e9 / (period / 1e3)
+        rate = rows * weight_bytes / 1e12 / (period / 1e3)     # two operations a two-byte weight
         print(f"bf16 prefill, {slots} slots x {chunk} tokens from context {context}: {period:.2f} ms "
-              f"of device time per call over 6 layers ({weight_bytes / 1e9:.2f} GB of bf16 weights "
-              f"= {roofline:.0f} GB/s; {wall:.2f} ms wall clock through the Python mirror); x10 for "
-              f"60 layers (extrapolated): {10 * period:.1f} ms, "
+              f"of device time per call over 6 layers and the K and V of a seventh "
+              f"({weight_bytes / 1e9:.2f} GB of bf16 weights x {rows} rows = {rate:.0f} TFLOP/s; "
+              f"{wall:.2f} ms wall clock through the Python mirror); x10 for 60 layers "
+              f"(extrapolated): {10 * period:.1f} ms, "
               f"{rows / (10 * period / 1e3):.0f} prompt tokens/s")
     runner.close()
 
 
 def prefill_prompt(launches=3, slots=24):
-    """Whole prompts from empty slots on one period of the 31B layer pattern: a lone 512-token
-    prompt and `slots` of them together (the rings stay unwrapped: a step takes up to 256 rows,
-    many eight-token pieces of one prompt), then a lone 3,072-token prompt and four of them
-    together (past the first 1,024 tokens the sliding layers go wave by wave). Wall clock through
-    the Python mirror, best of `launches`, and the same for ten periods (extrapolated)."""
+    """Whole prompts from empty slots on one period of the 31B layer pattern and a seventh layer (as
+    above; the step that ends a prompt runs its last row through it): a lone 512-token prompt and
+    `slots` of them together, then a lone 3,072-token prompt and four of them together (past the
+    sliding window), in packed steps of up to 2,048 rows. Wall clock through the Python mirror, best of
+    `launches`, and the same for ten periods (extrapolated)."""
     import time
-    config, runner, weight_bytes, keep = _period_model(slots, 3200, with_assistant=False)
+    config, runner, weight_bytes, keep = _period_model(slots, 3200, with_assistant=False,
+                                                       extra_layers=1)
     generator = torch.Generator().manual_seed(2)
     for count, length in ((1, 512), (slots, 512), (1, 3072), (4, 3072)):
         prompts = torch.randint(3, config.vocabulary_size, (count, length),

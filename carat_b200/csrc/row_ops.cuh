@@ -1,9 +1,9 @@
 // Row-wise fused operators of the verify / draft step. Each one produces a bf16 activation row the
 // way the reference does (same fp32 math, same bf16 rounding points) and, in the same launch,
 // quantises the whole [rows, width] tensor to e4m3 with the reference's tensor-wide scale rule
-// (amax / 448, cuda/linear.cu:76-115). The tensor-wide maximum couples all rows, so the kernels are
-// cooperative launches: one CTA per row, an atomic maximum, one grid barrier, then every CTA
-// quantises its row straight from shared memory. Nothing is re-read from HBM.
+// (amax / 448, cuda/linear.cu:76-115). The tensor-wide maximum couples all rows: one CTA per row (or
+// part of a row) keeps it in registers, an atomic maximum, one grid barrier, then every CTA quantises
+// what it holds. Nothing is re-read from HBM. Without a quantised target there is no barrier.
 #pragma once
 
 #include <cuda_runtime.h>
