@@ -299,8 +299,10 @@ int run_verify_attention(bool tensor_cores, const void *bf16_queries, const void
         (partials_need(long_chunk_keys) > partial_bytes ||
          score_rows * attention_chunks(a.max_cache_rows, long_chunk_keys) > stats_rows)) {
       // A stream under capture cannot get more scratch: it keeps to the uncut form's.
-      if (cudaStreamIsCapturing(cuda_stream, &capturing) != cudaSuccess)
+      if (cudaStreamIsCapturing(cuda_stream, &capturing) != cudaSuccess) {
+        capturing = cudaStreamCaptureStatusNone;
         cudaGetLastError();
+      }
       if (capturing != cudaStreamCaptureStatusNone)
         long_chunk_keys = uncut_chunk_rows;
     }
