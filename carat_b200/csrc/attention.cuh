@@ -106,18 +106,24 @@ inline int attention_chunks(int max_cache_rows, int chunk_keys) {
 // Cache rows per chunk of a long linear cache for the two-kernel tensor-core path. 1,024 where that
 // gives the SMs enough chunks: each costs a change of queries and a drain of the pipeline (24
 // contexts of 128 to 6,144: 512 to 768 rows are 6 % slower). A few requests leave most SMs without
-// a chunk of that size: they are cut into 256 to 512 rows when every chunk of the launch then still
-// has an SM to itself. Both kernels, cold L2, 32 / 4 heads of 512, five rows a request, us with the
-// rule and with 1,024 rows: one context of 1,000 42 and 58, of 3,000 44 and 58, of 8,000 50 and 58;
-// 500 to 2,000 six times 46 and 58. Where the rule stops: 900 twenty times (two chunks each would
-// not all find an SM) 60, 73 if cut; 5,000 four times (640 rows would fit) 62, 64 if cut.
+// a chunk of that size: contexts of more than 512 rows are cut into 256 to 512 when every chunk of
+// the launch then still has an SM to itself; into two, the least that a cut brings, only above 640
+// rows and on at most five sixths of the SMs. Both kernels and the sum of the chunks, five rows a
+// request, 32 / 4 heads of 512, back to back, us with the rule and with 1,024 rows: one context of
+// 560 25.9 and 31.6, of 1,020 25.9 and 43.4, of 4,500 29.1 and 46.1; five of 1,600 35.2 and 45.4;
+// twelve of 560 34.9 and 35.3, of 1,200 43.2 and 50.2; fifteen of 900, in two, 4 % faster (of 450
+// to 900 10 %). Beyond the rule: eight of 320 (29.7 cut and 27.1), eighteen of 640 (in two: 41.0
+// and 37.4; of 900 6 % slower), twenty of 900 (160 chunks on 148 SMs, cold: 73 and 60), four of
+// 5,000 (640 rows, cold: 64 and 62).
 // The cut follows the launch's number of requests and its longest context, so equal requests of one
 // launch are cut alike; in launches of another size the fp32 sums of a request may be taken in
 // another order.
 constexpr int uncut_chunk_rows = 1024;
 inline int chunk_rows(int requests, int kv_heads, int max_cache_rows, int multiprocessors) {
   const int chunks = multiprocessors / (requests * kv_heads);   // a request may have
-  if (chunks < 2)
+  if (chunks < 2 || max_cache_rows <= 512)
+    return uncut_chunk_rows;
+  if (chunks == 2 && (max_cache_rows <= 640 || 12 * requests * kv_heads > 5 * multiprocessors))
     return uncut_chunk_rows;
   const int rows = ((max_cache_rows + chunks - 1) / chunks + 127) / 128 * 128;
   return rows > 512 ? uncut_chunk_rows : rows < 256 ? 256 : rows;

@@ -80,7 +80,8 @@ public:
       require_cuda(cudaMemset(pointer_, 0, bytes_), "clear runner memory");
   }
   void release() {
-    cudaFree(pointer_);
+    if (pointer_ != nullptr)
+      cudaFree(pointer_);
     pointer_ = nullptr;
     bytes_ = 0;
   }
@@ -103,7 +104,8 @@ public:
     require_memory(cudaMallocHost(&pointer_, bytes), "allocate pinned mailbox");
   }
   void release() {
-    cudaFreeHost(pointer_);
+    if (pointer_ != nullptr)
+      cudaFreeHost(pointer_);
     pointer_ = nullptr;
   }
   template <typename T> T *get() const { return static_cast<T *>(pointer_); }

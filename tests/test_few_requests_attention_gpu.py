@@ -1,5 +1,5 @@
-"""Global attention of a few requests, whose contexts are cut into chunks of 256 to 512 rows while each
-chunk has an SM to itself, against the CUDA-core kernels (which do not cut by that rule), through the
+"""Global attention of a few requests, whose contexts of more than 512 rows are cut into chunks of 256 to
+512 while each chunk has an SM to itself, against the CUDA-core kernels (which do not cut by that rule), through the
 runner against the oracle, and under stream capture. The bar against the CUDA-core kernels is the one
 of the tensor-core attention's other comparisons: 2e-2 of the largest output."""
 import subprocess

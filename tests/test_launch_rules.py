@@ -62,6 +62,12 @@ def test_a_cut_context_leaves_every_chunk_an_sm(rules, sms):
                 assert chunk % 128 == 0 and (256 <= chunk <= 512 or chunk == 1024)
                 if chunk != 1024:
                     chunks = -(-rows // chunk)
+                    assert rows > 512
+                    if chunks == 2 and chunk > 256:
+                        assert rows > 640 and requests * kv_heads * 2 <= sms * 5 / 6
                     assert requests * kv_heads * chunks <= sms, (requests, kv_heads, rows)
     assert rules.chunk(20, 4, 905, sms) == 1024      # two chunks a request: 160 on 148 SMs
-    assert rules.chunk(1, 4, 905, sms) == 256
+    assert rules.chunk(18, 4, 905, sms) == 1024      # two chunks a request, on too many SMs
+    assert rules.chunk(13, 4, 905, sms) == 512 and rules.chunk(13, 4, 625, sms) == 1024
+    assert rules.chunk(8, 4, 325, sms) == 1024
+    assert rules.chunk(1, 4, 905, sms) == rules.chunk(5, 4, 565, sms) == 256
